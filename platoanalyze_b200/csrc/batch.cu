@@ -12,7 +12,10 @@
 #include <cmath>
 #include <vector>
 
+#include "fans.cuh"
 #include "plato_internal.cuh"
+
+int plato_create_unplanned(const plato_problem_desc* d, plato_problem** out);
 
 namespace plato {
 
@@ -172,11 +175,14 @@ int plato_create_batch(int32_t count, const plato_problem_desc* descs, plato_pro
     u.essential_bcs.values = bc_vals.empty() ? nullptr : bc_vals.data();
 
     plato_problem* h = nullptr;
-    if (int rc = plato_create(&u, &h)) return rc;
+    if (int rc = plato_create_unplanned(&u, &h)) return rc;
     h->batch.nseg = count;
     h->batch.node_off = node_off;
     h->batch.cell_off = cell_off;
-    if (int rc = setup_tiles(h)) {
+    int planned = fan_plan(h);
+    plan_pool_close(h);
+    if (!planned) planned = setup_tiles(h);
+    if (int rc = planned) {
         const std::string msg = h->last_error;
         plato_destroy(h);
         return plato_fail(nullptr, rc, msg);

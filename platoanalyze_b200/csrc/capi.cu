@@ -8,6 +8,7 @@
 #include <mutex>
 #include <utility>
 
+#include "fans.cuh"
 #include "plato_internal.cuh"
 
 namespace plato {
@@ -15,7 +16,7 @@ int build_graph(plato_problem* h);
 int launch_internal_force(plato_problem* h, const double* u, const double* z, double* R, double scale_F);
 int launch_traction(plato_problem* h, int32_t nfaces, const int32_t* fcell, const int32_t* floc, const double t[3]);
 int launch_nodal_control_derivative(plato_problem* h, int mode, const double* u, const double* z,
-                                    const double* lam, double* cellbuf, double* out, int accumulate);
+                                    const double* lam, double* out, int accumulate);
 int launch_energy(plato_problem* h, const double* u, const double* z, double* result);
 int launch_energy_and_gradient(plato_problem* h, const double* u, const double* z, double* result, double* dfdz);
 int launch_assemble_jacobian(plato_problem* h, const double* z, double* entries);
@@ -37,10 +38,9 @@ int matfree_rhs(plato_problem* h, double* b, double scale);
 int launch_dirichlet_rhs(plato_problem* h, double* rhs, double scale);
 int launch_ebe_apply64_unmasked(plato_problem* h, const double* x, double* y);
 int launch_masked_axpy(plato_problem* h, double a, const double* x, double* y);
-int matfree_setup(plato_problem* h, const double* z);
-int launch_ebe_apply64(plato_problem* h, const double* x, double* y, const PcgScalars* S);
-int launch_mask_copy(plato_problem* h, const double* x, double* y);
+int launch_constrained_apply(plato_problem* h, const double* z, const double* x, double* y);
 int launch_sell_spmv(plato_problem* h, const double* vals, const double* x, double* y);
+int launch_coords_soa(plato_problem* h);
 int launch_volume(plato_problem* h, const Material& pen, const double* z, double* result);
 int launch_volume_gradient(plato_problem* h, const Material& pen, const double* z, double* dvdz);
 }  // namespace plato
@@ -134,6 +134,34 @@ int check_opts(plato_problem* h, const plato_solver_opts& o) {
 }  // namespace
 
 extern "C" {
+static int create_handle(const plato_problem_desc* d, plato_problem** out);
+}
+
+// A handle whose element kernels are not planned yet (a batch knows its members only later, a
+// filter has no use for the plan); the caller plans and closes the set-up's pool.
+int plato_create_unplanned(const plato_problem_desc* d, plato_problem** out) { return create_handle(d, out); }
+
+namespace plato {
+int plan_pool_open(plato_problem* h) {
+    if (h->plan_pool) return PLATO_OK;
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = h->device;
+    PLATO_CUDA(h, cudaMemPoolCreate(&h->plan_pool, &props));
+    uint64_t all = UINT64_MAX;
+    PLATO_CUDA(h, cudaMemPoolSetAttribute(h->plan_pool, cudaMemPoolAttrReleaseThreshold, &all));
+    return PLATO_OK;
+}
+void plan_pool_close(plato_problem* h) {
+    if (!h->plan_pool) return;
+    cudaStreamSynchronize(h->stream);
+    cudaMemPoolDestroy(h->plan_pool);
+    h->plan_pool = nullptr;
+}
+}  // namespace plato
+
+extern "C" {
 
 const char* plato_last_error(const plato_problem* h) {
     return h ? h->last_error.c_str() : g_create_error.c_str();
@@ -142,12 +170,13 @@ const char* plato_last_error(const plato_problem* h) {
 int plato_destroy(plato_problem* h) {
     if (!h) return PLATO_OK;
     cudaStreamSynchronize(h->stream);
-    dfree(h->conn); dfree(h->coords); dfree(h->row_map); dfree(h->cols); dfree(h->diag);
+    plan_pool_close(h);
+    dfree(h->conn); dfree(h->coords); dfree(h->coords_soa); dfree(h->row_map); dfree(h->cols); dfree(h->diag);
     dfree(h->n2c_ptr); dfree(h->n2c); dfree(h->F); dfree(h->bc_dofs); dfree(h->bc_values);
     dfree(h->asm_plan); dfree(h->asm_wide); dfree(h->asm_mirror); dfree(h->asm_wideflag); dfree(h->ritz_small);
     dfree(h->bc_mask); dfree(h->K); dfree(h->KT); dfree(h->v_r); dfree(h->v_z); dfree(h->v_p);
     dfree(h->v_Ap); dfree(h->v_dinv); dfree(h->v_b); dfree(h->v_x); dfree(h->v_tmp);
-    dfree(h->partials); dfree(h->cellbuf); dfree(h->scal); dfree(h->red_out); dfree(h->red_ticket);
+    dfree(h->partials); dfree(h->scal); dfree(h->red_out); dfree(h->red_ticket);
     dfree(h->f_r); dfree(h->f_z); dfree(h->f_p); dfree(h->f_Ap); dfree(h->f_x); dfree(h->f_dinv);
     dfree(h->f_K); dfree(h->h_K); dfree(h->f_coords); dfree(h->f_z_ctrl); dfree(h->d_z_ctrl);
     dfree(h->d_z_in); dfree(h->d_u_out); dfree(h->d_g_out);
@@ -156,7 +185,8 @@ int plato_destroy(plato_problem* h) {
     if (h->sell16) cudaFree(h->sell16);
     if (h->sell16s) cudaFree(h->sell16s);
     dfree(h->f_sq); dfree(h->f_isq);
-    dfree(h->mf_w64); dfree(h->mf_w32); dfree(h->v_q);
+    dfree(h->v_q);
+    fan_release(h);
     dfree(h->f_res); dfree(h->f_d0); dfree(h->f_d1); dfree(h->f_y); dfree(h->f_w);
     dfree(h->wave_flags); dfree(h->wave_ctl); dfree(h->lanczos);
     for (int32_t*& o : h->wave_order) dfree(o);
@@ -176,7 +206,7 @@ int plato_destroy(plato_problem* h) {
     return PLATO_OK;
 }
 
-int plato_create(const plato_problem_desc* d, plato_problem** out) {
+static int create_handle(const plato_problem_desc* d, plato_problem** out) {
     if (!out) return plato_fail(nullptr, PLATO_BAD_INPUT, "null output handle pointer");
     *out = nullptr;
     if (!d) return plato_fail(nullptr, PLATO_BAD_INPUT, "null problem description");
@@ -242,6 +272,9 @@ int plato_create(const plato_problem_desc* d, plato_problem** out) {
     CRC(dmalloc(h, &h->coords, n));
     CCUDA(cudaMemcpy(h->conn, m.connectivity, sizeof(int4) * size_t(h->C), cudaMemcpyHostToDevice));
     CCUDA(cudaMemcpy(h->coords, m.coords, sizeof(double) * size_t(n), cudaMemcpyHostToDevice));
+    CRC(dmalloc(h, &h->coords_soa, n));
+    CRC(launch_coords_soa(h));
+    CRC(plan_pool_open(h));
     CRC(build_graph(h));
     CRC(build_sell_pattern(h));
 
@@ -273,7 +306,6 @@ int plato_create(const plato_problem_desc* d, plato_problem** out) {
         CRC(dmalloc(h, v, n));
     h->partials_len = 148 * 64;
     CRC(dmalloc(h, &h->partials, 4 * int64_t(h->partials_len)));
-    CRC(dmalloc(h, &h->cellbuf, h->C));
     CRC(dmalloc(h, &h->scal, 1));
     CRC(dmalloc(h, &h->red_out, 4));  // up to 4 reduction results
     CRC(dmalloc(h, &h->red_ticket, 1));
@@ -311,6 +343,19 @@ int plato_create(const plato_problem_desc* d, plato_problem** out) {
 #undef CCUDA
     *out = h;
     return PLATO_OK;
+}
+
+int plato_create(const plato_problem_desc* d, plato_problem** out) {
+    int rc = plato_create_unplanned(d, out);
+    if (rc) return rc;
+    rc = fan_plan(*out);
+    plan_pool_close(*out);
+    if (rc) {
+        g_create_error = (*out)->last_error;
+        plato_destroy(*out);
+        *out = nullptr;
+    }
+    return rc;
 }
 
 int plato_set_stream(plato_problem* h, void* stream) {
@@ -488,7 +533,7 @@ int plato_vf_gradient_z(plato_problem* h, const double* u, const double* z, doub
 
 int plato_vf_gradient_z_apply(plato_problem* h, const double* u, const double* z, const double* lam, double* out) {
     NEED(h, u && z && lam && out, "null device pointer");
-    return launch_nodal_control_derivative(h, 3, u, z, lam, h->cellbuf, out, 1);
+    return launch_nodal_control_derivative(h, 3, u, z, lam, out, 1);
 }
 
 int plato_sf_value(plato_problem* h, const double* u, const double* z, double* value) {
@@ -508,7 +553,7 @@ int plato_sf_gradient_u(plato_problem* h, const double* u, const double* z, doub
 
 int plato_sf_gradient_z(plato_problem* h, const double* u, const double* z, double* dfdz) {
     NEED(h, u && z && dfdz, "null device pointer");
-    return launch_nodal_control_derivative(h, 1, u, z, nullptr, h->cellbuf, dfdz, 0);
+    return launch_nodal_control_derivative(h, 1, u, z, nullptr, dfdz, 0);
 }
 
 static Material volume_penalty(const plato_penalty* p, const plato_problem* h) {
@@ -548,11 +593,7 @@ int plato_matvec_plus(plato_problem* h, int32_t rb, int32_t cb, const double* en
 
 int plato_apply_operator(plato_problem* h, const double* z, int32_t operator_kind, const double* x, double* y) {
     NEED(h, z && x && y, "null device pointer");
-    if (operator_kind == PLATO_OPERATOR_MATRIX_FREE) {
-        RC(matfree_setup(h, z));
-        RC(launch_ebe_apply64(h, x, y, nullptr));
-        return launch_mask_copy(h, x, y);
-    }
+    if (operator_kind == PLATO_OPERATOR_MATRIX_FREE) return launch_constrained_apply(h, z, x, y);
     if (operator_kind != PLATO_OPERATOR_ASSEMBLED) return plato_fail(h, PLATO_BAD_INPUT, "unknown operator_kind");
     RC(dmalloc(h, &h->K, 9 * h->nblocks));
     RC(launch_assemble_jacobian(h, z, h->K));
@@ -659,7 +700,7 @@ int plato_problem_criterion_gradient(plato_problem* h, const double* z, const do
         // lambda = -u (src/elliptic/Problem.hpp:423-427): dfdz + (dR/dz)^T lambda fused per cell
         st->iterations = 0; st->refinements = 0; st->relative_residual = 0.0; st->converged = 1; st->status = 0;
         RC(elem_time_begin(h, 2));
-        RC(launch_nodal_control_derivative(h, 2, u, z, nullptr, h->cellbuf, dfdz, 0));
+        RC(launch_nodal_control_derivative(h, 2, u, z, nullptr, dfdz, 0));
         return elem_time_end(h, 2);
     }
     // adjoint: K^T lambda = -df/du with zero-valued constraints (Problem.hpp:429-441, 701-713)
@@ -667,7 +708,7 @@ int plato_problem_criterion_gradient(plato_problem* h, const double* z, const do
     RC(launch_internal_force(h, u, z, h->v_tmp, 0.0));
     RC(launch_axpby(h, n, -1.0, h->v_tmp, 0.0, h->v_tmp));
     RC(solve_adjoint(h, z, h->v_tmp, h->v_x, st));
-    return launch_nodal_control_derivative(h, 4, u, z, h->v_x, h->cellbuf, dfdz, 0);
+    return launch_nodal_control_derivative(h, 4, u, z, h->v_x, dfdz, 0);
 }
 
 int plato_problem_solve_and_gradient_host(plato_problem* h, const double* z_host, const double* u0_host,

@@ -96,7 +96,7 @@ int build_graph(plato_problem* h) {
 
     // connectivity sanity (ids in range, 4 distinct nodes per cell)
     int32_t* d_bad = nullptr;
-    PLATO_CUDA(h, cudaMallocAsync(&d_bad, sizeof(int32_t), s));
+    PLATO_CUDA(h, plan_alloc(h, &d_bad, sizeof(int32_t), s));
     PLATO_CUDA(h, cudaMemsetAsync(d_bad, 0, sizeof(int32_t), s));
     k_check_conn<<<grid_for(C, T), T, 0, s>>>(C, N, h->conn, d_bad);
     PLATO_LAUNCH_CHECK(h);
@@ -110,9 +110,9 @@ int build_graph(plato_problem* h) {
     const int64_t npairs = 16 * (int64_t)C + N;
     uint64_t *k_in = nullptr, *k_out = nullptr, *k_uniq = nullptr;
     int64_t* d_num = nullptr;
-    PLATO_CUDA(h, cudaMallocAsync(&k_in, npairs * sizeof(uint64_t), s));
-    PLATO_CUDA(h, cudaMallocAsync(&k_out, npairs * sizeof(uint64_t), s));
-    PLATO_CUDA(h, cudaMallocAsync(&d_num, sizeof(int64_t), s));
+    PLATO_CUDA(h, plan_alloc(h, &k_in, npairs * sizeof(uint64_t), s));
+    PLATO_CUDA(h, plan_alloc(h, &k_out, npairs * sizeof(uint64_t), s));
+    PLATO_CUDA(h, plan_alloc(h, &d_num, sizeof(int64_t), s));
     k_pair_keys<<<grid_for(npairs, T, 148 * 64), T, 0, s>>>(C, N, h->conn, k_in);
     PLATO_LAUNCH_CHECK(h);
     const int ebits = 32 + end_bit_for(N);
@@ -121,7 +121,7 @@ int build_graph(plato_problem* h) {
     PLATO_CUDA(h, cub::DeviceSelect::Unique(nullptr, tmp_uniq, k_out, k_in, d_num, npairs, s));
     void* tmp = nullptr;
     const size_t tmp_bytes = tmp_sort > tmp_uniq ? tmp_sort : tmp_uniq;
-    PLATO_CUDA(h, cudaMallocAsync(&tmp, tmp_bytes, s));
+    PLATO_CUDA(h, plan_alloc(h, &tmp, tmp_bytes, s));
     size_t tb = tmp_bytes;
     PLATO_CUDA(h, cub::DeviceRadixSort::SortKeys(tmp, tb, k_in, k_out, npairs, 0, ebits, s));
     tb = tmp_bytes;
@@ -142,7 +142,7 @@ int build_graph(plato_problem* h) {
     // ---- node -> (cell, slot) incidence ----------------------------------------------
     const int64_t ninc = 4 * (int64_t)C;
     int32_t* counts = nullptr;
-    PLATO_CUDA(h, cudaMallocAsync(&counts, (N + 1) * sizeof(int32_t), s));
+    PLATO_CUDA(h, plan_alloc(h, &counts, (N + 1) * sizeof(int32_t), s));
     PLATO_CUDA(h, cudaMemsetAsync(counts, 0, (N + 1) * sizeof(int32_t), s));
     k_incidence_keys<<<grid_for(ninc, T, 148 * 64), T, 0, s>>>(C, h->conn, k_in, counts);
     PLATO_LAUNCH_CHECK(h);

@@ -24,6 +24,8 @@
 
 #include "plato_internal.cuh"
 
+int plato_create_unplanned(const plato_problem_desc* d, plato_problem** out);
+
 namespace plato {
 
 MeshView mesh_view(const plato_problem* h);
@@ -239,7 +241,8 @@ int plato_create_helmholtz(const plato_helmholtz_desc* desc, plato_problem** out
     d.solver.chebyshev_degree = 0;
     d.solver.coarse_cells[0] = d.solver.coarse_cells[1] = d.solver.coarse_cells[2] = 0;
     plato_problem* h = nullptr;
-    if (int rc = plato_create(&d, &h)) return rc;
+    if (int rc = plato_create_unplanned(&d, &h)) return rc;
+    plan_pool_close(h);
     h->physics = 1;
     h->helm_length = L;
     h->helm_surface = alpha;

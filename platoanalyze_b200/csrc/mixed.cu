@@ -42,7 +42,6 @@ int launch_sell_scale16(plato_problem* h, const double* sell64, const double* di
 int launch_sell_spmv(plato_problem* h, const double* vals, const double* x, double* y);
 int launch_ebe_apply64(plato_problem* h, const double* x, double* y, const PcgScalars* S);
 int launch_ebe_apply32(plato_problem* h, const float* x, float* y, const PcgScalars* S);
-int launch_mask_copy(plato_problem* h, const double* x, double* y);
 int matfree_setup(plato_problem* h, const double* z);
 SellView sell_view(const plato_problem* h);
 int spmv_blocks(const plato_problem* h);
@@ -1194,11 +1193,7 @@ int fcg_poly(plato_problem* h, const double* b, double* x, plato_solve_stats* st
     bool coarse_waited = false;
 
     auto outer_apply = [&](const double* in, double* out) -> int {
-        if (mf) {
-            int r2 = launch_ebe_apply64(h, in, out, nullptr);
-            if (r2) return r2;
-            return launch_mask_copy(h, in, out);
-        }
+        if (mf) return launch_ebe_apply64(h, in, out, nullptr);
         return launch_sell_spmv(h, h->sell64, in, out);
     };
     const bool coarse = h->coarse.active != 0;

@@ -135,6 +135,25 @@ struct BatchState {
     std::vector<plato_solve_stats> last;  // per-member statistics of the last solve
 };
 
+// Cells grouped into fans and tiles for the element kernels (fans.cu, once per mesh; the arrays
+// are described in fans.cuh) and those kernels' workspaces.
+constexpr int kFanMaxCtas = 148 * 32;  // CTAs of an element kernel
+struct FanPlan {
+    int       ready = 0;
+    int32_t   nfans = 0, ntiles = 0, width = 0;
+    int32_t*  rec = nullptr;
+    int32_t*  cells = nullptr;
+    int32_t*  tile_ptr = nullptr;
+    uint32_t* place = nullptr;
+    int32_t*  slot = nullptr;
+    uint16_t* inc = nullptr;
+    int32_t*  node_ptr = nullptr;
+    double*   part = nullptr;  // [3 * entries] node sums of each tile
+    double*   sums = nullptr;  // [kFanMaxCtas] block sums of the criteria
+    double*   w64 = nullptr;   // [6 * nfans] SIMP weight of each cell (matrix-free operator)
+    float*    w32 = nullptr;   // the same in FP32
+};
+
 // Two-level preconditioner state (coarse.cu).
 struct CoarseSpace {
     int      nc[3] = {0, 0, 0};   // coarse cells per axis
@@ -189,6 +208,8 @@ struct plato_problem {
     // mesh
     int4*   conn = nullptr;
     double* coords = nullptr;
+    double* coords_soa = nullptr;  // x, y, z planes: a warp that reads consecutive nodes touches 3 cache lines
+                                   // per component instead of 7 (the element kernels are bound by that)
     // graph
     int32_t* row_map = nullptr;
     int32_t* cols = nullptr;
@@ -226,7 +247,6 @@ struct plato_problem {
     double* v_x = nullptr;
     double* v_tmp = nullptr;
     double* partials = nullptr;    // block partial sums of reductions
-    double* cellbuf = nullptr;     // one double per cell (per-cell quantities before a nodal sum)
     int32_t partials_len = 0;
     PcgScalars* scal = nullptr;    // device
     PcgScalars* scal_host = nullptr;  // pinned mirror
@@ -260,9 +280,9 @@ struct plato_problem {
     void*   sell16s = nullptr;     // FP16 entries of D^-1/2 A D^-1/2 (scaled mixed precision)
     float*  f_sq = nullptr;        // D^1/2 (scaled mixed precision)
     float*  f_isq = nullptr;       // D^-1/2
-    // matrix-free operator data (matfree.cu) and mixed-precision work vectors (mixed.cu)
-    double* mf_w64 = nullptr;      // per-cell SIMP weight s(rho_e), FP64
-    float*  mf_w32 = nullptr;      // same, FP32
+    FanPlan fans{};                // cells grouped for the element kernels (fans.cu)
+    cudaMemPool_t plan_pool = nullptr;  // scratch of the mesh-level set-up, while that runs
+    // mixed-precision work vectors (mixed.cu)
     double* v_q = nullptr;         // A p of the flexible CG
     float*  f_res = nullptr;       // Chebyshev residual
     float*  f_d0 = nullptr;        // Chebyshev directions (double buffered)
@@ -385,6 +405,17 @@ int ensure_smem_attribute(plato_problem* h, const void* kernel, int bytes);
 
 namespace plato {
 
+// Scratch of the mesh-level set-up (graph, SELL pattern, fans) comes from a pool of its own that
+// keeps what is freed until the set-up ends: from the default pool every synchronisation would give
+// it back to the system, and mapping it again costs more than the sorts that use it.
+int plan_pool_open(plato_problem* h);
+void plan_pool_close(plato_problem* h);
+template <typename T>
+inline cudaError_t plan_alloc(plato_problem* h, T** p, size_t bytes, cudaStream_t s) {
+    return h->plan_pool ? cudaMallocFromPoolAsync(reinterpret_cast<void**>(p), bytes, h->plan_pool, s)
+                        : cudaMallocAsync(reinterpret_cast<void**>(p), bytes, s);
+}
+
 constexpr int kNumSMs = 148;
 
 inline int grid_for(int64_t n, int threads, int64_t max_blocks = 148 * 32) {
@@ -496,14 +527,15 @@ __device__ __forceinline__ T ipow(T r, int p) {
 
 template <typename T>
 __device__ __forceinline__ T simp(const Material& m, T rho) {
-    const T pw = m.p_int >= 0 ? ipow(rho, m.p_int) : T(pow(double(rho), m.p));
+    const T pw = m.p_int == 3 ? rho * rho * rho : (m.p_int >= 0 ? ipow(rho, m.p_int) : T(pow(double(rho), m.p)));
     return T(m.rho_min) + (T(1) - T(m.rho_min)) * pw;
 }
 
 template <typename T>
 __device__ __forceinline__ T simp_dx(const Material& m, T rho) {
     T pw;
-    if (m.p_int >= 1) pw = ipow(rho, m.p_int - 1);
+    if (m.p_int == 3) pw = rho * rho;
+    else if (m.p_int >= 1) pw = ipow(rho, m.p_int - 1);
     else if (m.p_int == 0) pw = T(0);
     else pw = T(pow(double(rho), m.p - 1.0));
     return (T(1) - T(m.rho_min)) * (T(m.p) * pw);

@@ -188,22 +188,22 @@ int build_sell_pattern(plato_problem* h) {
     PLATO_CUDA(h, cudaMalloc(&P.ptr, sizeof(int64_t) * (ns + 1)));
     int64_t* slots = nullptr;
     int32_t* slice_nnz = nullptr;
-    PLATO_CUDA(h, cudaMallocAsync(&slots, sizeof(int64_t) * (ns + 1), s));
-    PLATO_CUDA(h, cudaMallocAsync(&slice_nnz, sizeof(int32_t) * ns, s));
+    PLATO_CUDA(h, plan_alloc(h, &slots, sizeof(int64_t) * (ns + 1), s));
+    PLATO_CUDA(h, plan_alloc(h, &slice_nnz, sizeof(int32_t) * ns, s));
     PLATO_CUDA(h, cudaMemsetAsync(slots, 0, sizeof(int64_t) * (ns + 1), s));
     k_slice_width<<<grid_for((int64_t)ns * 32, 256), 256, 0, s>>>(N, ns, h->row_map, P.width, slots, slice_nnz);
     PLATO_LAUNCH_CHECK(h);
     size_t tb = 0;
     PLATO_CUDA(h, cub::DeviceScan::ExclusiveSum(nullptr, tb, slots, P.ptr, ns + 1, s));
     void* tmp = nullptr;
-    PLATO_CUDA(h, cudaMallocAsync(&tmp, tb, s));
+    PLATO_CUDA(h, plan_alloc(h, &tmp, tb, s));
     PLATO_CUDA(h, cub::DeviceScan::ExclusiveSum(tmp, tb, slots, P.ptr, ns + 1, s));
     size_t tb2 = 0;
     int32_t* d_max = nullptr;
-    PLATO_CUDA(h, cudaMallocAsync(&d_max, sizeof(int32_t), s));
+    PLATO_CUDA(h, plan_alloc(h, &d_max, sizeof(int32_t), s));
     PLATO_CUDA(h, cub::DeviceReduce::Max(nullptr, tb2, slice_nnz, d_max, ns, s));
     void* tmp2 = nullptr;
-    PLATO_CUDA(h, cudaMallocAsync(&tmp2, tb2, s));
+    PLATO_CUDA(h, plan_alloc(h, &tmp2, tb2, s));
     PLATO_CUDA(h, cub::DeviceReduce::Max(tmp2, tb2, slice_nnz, d_max, ns, s));
     int32_t maxnnz = 0;
     PLATO_CUDA(h, cudaMemcpyAsync(&P.total_slots, P.ptr + ns, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
