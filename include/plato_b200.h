@@ -127,7 +127,9 @@ typedef struct plato_solver_opts {
                                  per launch.  0 or 1 = one launch per step; 2..16 = that many
                                  steps in one launch, each (step, 512-row tile) task waiting only
                                  for the tiles of the step before that its columns reach, so the
-                                 matrix can be re-read from L2 (needs 16-bit column offsets)  */
+                                 matrix can be re-read from L2 (needs 16-bit column offsets).
+                                 Systems of up to some 75,000 nodes run their iterations in
+                                 cooperative launches instead, whatever this says             */
     int32_t sweep_lag;        /* multi-step sweep: tiles of 512 rows by which each step trails the
                                  one before beyond the column reach (0 = 600 / sweep_steps)  */
 } plato_solver_opts;
@@ -195,7 +197,7 @@ int plato_reset_instrumentation(plato_problem* h);
  * kind 2 = the Jacobian assembly of each assembled solve, kind 3 = the Galerkin product of
  * the two-level coarse operator, kind 4 = its dense factorization and inverse (kinds 3 and 4
  * count coarse operator set-ups); kinds 5-8 time every call with timing on: 5 = the residual
- * of plato_vf_value (load copy + element force kernel), 6 = the energy sum of plato_sf_value,
+ * of plato_vf_value (load copy + element force kernels), 6 = the energy sum of plato_sf_value,
  * 7 = the self-adjoint dC/dz of plato_problem_criterion_gradient (per-cell pass + nodal
  * sums), 8 = plato_problem_criterion_value_and_gradient's one pass (+ nodal sums).  Reading
  * kinds 5-8 waits for the last timed launch of that kind.  With the multi-step FP16 sweep

@@ -187,6 +187,7 @@ int plato_destroy(plato_problem* h) {
     dfree(h->f_sq); dfree(h->f_isq);
     dfree(h->v_q);
     fan_release(h);
+    if (h->grid_box) cudaFree(h->grid_box);
     dfree(h->f_res); dfree(h->f_d0); dfree(h->f_d1); dfree(h->f_y); dfree(h->f_w);
     dfree(h->wave_flags); dfree(h->wave_ctl); dfree(h->lanczos);
     for (int32_t*& o : h->wave_order) dfree(o);

@@ -26,6 +26,7 @@
 
 #include <cub/cub.cuh>
 
+#include "coarse_view.cuh"
 #include "plato_internal.cuh"
 
 namespace plato {
@@ -36,34 +37,6 @@ namespace {
 
 constexpr int kBatch = 32;     // elements staged per Galerkin batch (8 threads each)
 constexpr int kThreadsPerCta = 256;
-
-struct CoarseView {
-    int nc0, nc1, nc2;
-    double x0, y0, z0, hx, hy, hz;
-    double ihx, ihy, ihz;  // 1 / h: local coordinates of the hot kernels are (x - lo) * ih
-};
-
-__host__ __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
-
-__device__ __forceinline__ void cell_of(const CoarseView& cv, double x, double y, double z, int& cx, int& cy,
-                                        int& cz) {
-    cx = clampi(int(floor((x - cv.x0) / cv.hx)), 0, cv.nc0 - 1);
-    cy = clampi(int(floor((y - cv.y0) / cv.hy)), 0, cv.nc1 - 1);
-    cz = clampi(int(floor((z - cv.z0) / cv.hz)), 0, cv.nc2 - 1);
-}
-
-__device__ __forceinline__ int cell_id(const CoarseView& cv, int cx, int cy, int cz) {
-    return (cx * cv.nc1 + cy) * cv.nc2 + cz;
-}
-
-__device__ __forceinline__ int coarse_node(const CoarseView& cv, int ix, int iy, int iz) {
-    return (ix * (cv.nc1 + 1) + iy) * (cv.nc2 + 1) + iz;
-}
-
-// trilinear weight of corner (bx,by,bz) at local coordinates (u,v,w)
-__device__ __forceinline__ double corner_weight(int b, double u, double v, double w) {
-    return ((b & 4) ? u : 1.0 - u) * ((b & 2) ? v : 1.0 - v) * ((b & 1) ? w : 1.0 - w);
-}
 
 __global__ void k_node_keys(int32_t N, const double* __restrict__ coords, CoarseView cv, uint32_t* __restrict__ key,
                             int32_t* __restrict__ val, int32_t* __restrict__ count) {
@@ -786,42 +759,11 @@ k_restrict_cells(CoarseView cv, int split, const int32_t* __restrict__ node_ptr,
             for (int d = 0; d < 3; ++d) s[3 * b + d] += wgt * val[d];
         }
     }
-    // warp sums of the 24 values by halving: each exchange hands half of a lane's values to its
-    // partner, so after offsets 16, 8, 4 a lane holds 3 of the 24 sums (which 3 set by lane bits
-    // 4..2) and offsets 2, 1 finish them -- 27 shuffles instead of 24 x 5
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double t12[12], t6[6], t3[3];
-    {
-        const bool hi = (lane & 16) != 0;
-#pragma unroll
-        for (int i = 0; i < 12; ++i) {
-            const double send = hi ? s[i] : s[12 + i];
-            t12[i] = (hi ? s[12 + i] : s[i]) + __shfl_xor_sync(0xffffffffu, send, 16);
-        }
-    }
-    {
-        const bool hi = (lane & 8) != 0;
-#pragma unroll
-        for (int i = 0; i < 6; ++i) {
-            const double send = hi ? t12[i] : t12[6 + i];
-            t6[i] = (hi ? t12[6 + i] : t12[i]) + __shfl_xor_sync(0xffffffffu, send, 8);
-        }
-    }
-    {
-        const bool hi = (lane & 4) != 0;
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            const double send = hi ? t6[i] : t6[3 + i];
-            t3[i] = (hi ? t6[3 + i] : t6[i]) + __shfl_xor_sync(0xffffffffu, send, 4);
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        t3[i] += __shfl_xor_sync(0xffffffffu, t3[i], 2);
-        t3[i] += __shfl_xor_sync(0xffffffffu, t3[i], 1);
-    }
+    double t3[3];
+    warp_sum24(s, lane, t3);
     if ((lane & 3) == 0) {
-        const int base = ((lane & 16) ? 12 : 0) + ((lane & 8) ? 6 : 0) + ((lane & 4) ? 3 : 0);
+        const int base = warp_sum24_first(lane);
 #pragma unroll
         for (int i = 0; i < 3; ++i) sh[wid][base + i] = t3[i];
     }
@@ -949,7 +891,7 @@ __global__ void k_prolong(int32_t N, CoarseView cv, const double* __restrict__ c
 
 }  // namespace
 
-static CoarseView coarse_view(const plato_problem* h) {
+CoarseView coarse_view(const plato_problem* h) {
     const CoarseSpace& c = h->coarse;
     return CoarseView{c.nc[0], c.nc[1], c.nc[2], c.x0[0], c.x0[1], c.x0[2], c.h[0], c.h[1], c.h[2],
                       1.0 / c.h[0], 1.0 / c.h[1], 1.0 / c.h[2]};

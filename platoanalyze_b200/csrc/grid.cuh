@@ -1,0 +1,115 @@
+// Grid-wide sums and barriers of the cooperative Krylov kernels (pcg_grid.cu, fcg_grid.cu).
+#pragma once
+
+#include "solver_common.cuh"
+
+namespace plato {
+
+// A grid-wide sum: every CTA writes its block sums to its place of a box, adds one to a counter
+// (release), and one of its threads waits until the counter has reached the number of CTAs times the
+// number of this barrier (acquire); then all CTAs read the box and add it in CTA order, so all of
+// them get the same bits.  Two boxes alternate: a CTA that writes barrier n + 2 has seen everyone at
+// n + 1, hence done with reading n.  One waiting thread per CTA keeps the counter's cache line free for
+// the arrivals; with every CTA polling every other's place, 80 CTAs took 2.6 us longer per barrier
+// than 8.  Every wait has a limit; when one runs out the CTA raises `abort`, all CTAs leave, and the
+// host goes on with the launch-per-stage loop from the x that is there.
+constexpr uint32_t kGridPolls = 1u << 22;  // a second or two
+constexpr int kGridValues = 2;             // values of one sum at most
+constexpr int kGridSmemMax = 224 * 1024;   // dynamic shared memory: the opt-in limit less the static arrays
+
+struct GridBox {
+    double*   box;    // [2][kGridValues][gridDim.x]
+    uint32_t* count;  // arrivals in this launch
+    int32_t*  abort;
+};
+
+// acquire-release at GPU scope; __threadfence() is the sequentially consistent one, which costs more
+__device__ __forceinline__ void grid_fence() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+
+// Thread 0 of a CTA whose other threads' writes a __syncthreads() has put before this.
+__device__ __forceinline__ bool grid_arrive_and_wait(const GridBox& a, uint32_t barrier) {
+    const uint32_t target = barrier * gridDim.x;
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.count) : "memory");
+    for (uint32_t polls = 1;; ++polls) {
+        uint32_t v;
+        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.count) : "memory");
+        if (int32_t(v - target) >= 0) break;
+        if (polls > kGridPolls || ((polls & 1023u) == 0 && *reinterpret_cast<volatile int32_t*>(a.abort))) {
+            *reinterpret_cast<volatile int32_t*>(a.abort) = 1;
+            return false;
+        }
+    }
+    grid_fence();
+    return true;
+}
+
+// Sums NV values over the grid (the same bits in every thread) and orders all global writes before
+// it ahead of all reads after it.  `barrier` counts the barriers of the launch from 1.  False when a wait
+// ran out or another CTA gave up.
+template <int NV>
+__device__ __forceinline__ bool grid_sum(double (&v)[NV], const GridBox& a, uint32_t barrier, double (*sh_cta)[32],
+                                         double (*sh_grid)[32]) {
+    const int tid = threadIdx.x, w = tid >> 5, l = tid & 31, G = gridDim.x;
+#pragma unroll
+    for (int q = 0; q < NV; ++q) v[q] = warp_sum(v[q]);
+    if (l == 0)
+#pragma unroll
+        for (int q = 0; q < NV; ++q) sh_cta[q][w] = v[q];
+    __syncthreads();
+    double* box = a.box + (barrier & 1u) * kGridValues * G;
+    bool ok = true;
+    if (w == 0) {
+        const int nw = blockDim.x >> 5;
+#pragma unroll
+        for (int q = 0; q < NV; ++q) v[q] = warp_sum(l < nw ? sh_cta[q][l] : 0.0);
+        if (l == 0) {
+#pragma unroll
+            for (int q = 0; q < NV; ++q) *reinterpret_cast<volatile double*>(box + q * G + blockIdx.x) = v[q];
+            ok = grid_arrive_and_wait(a, barrier);
+        }
+    }
+    if (__syncthreads_or(!ok)) return false;
+    double got[NV];
+#pragma unroll
+    for (int q = 0; q < NV; ++q) got[q] = warp_sum(tid < G ? *reinterpret_cast<volatile double*>(box + q * G + tid) : 0.0);
+    if (l == 0)
+#pragma unroll
+        for (int q = 0; q < NV; ++q) sh_grid[q][w] = got[q];
+    __syncthreads();
+    const int nw = (G + 31) >> 5;  // the grid has no more CTAs than a CTA has threads
+#pragma unroll
+    for (int q = 0; q < NV; ++q) {
+        v[q] = 0.0;
+        for (int i = 0; i < nw; ++i) v[q] += sh_grid[q][i];
+    }
+    return true;
+}
+
+// The same without values: every write before it in the grid is seen by every read after it.
+__device__ __forceinline__ bool grid_barrier(const GridBox& a, uint32_t barrier) {
+    __syncthreads();
+    const bool ok = threadIdx.x != 0 || grid_arrive_and_wait(a, barrier);
+    return !__syncthreads_or(!ok);
+}
+
+// Cooperative launch of one CTA per SM.
+template <typename Args>
+inline cudaError_t launch_cooperative(void (*kernel)(Args), int grid, int block, size_t smem, cudaStream_t stream,
+                                      const Args& args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(unsigned(grid));
+    cfg.blockDim = dim3(unsigned(block));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args);
+}
+
+// The boxes, counter (cleared for the next launch) and abort flag of a handle (pcg_grid.cu).
+int grid_box(plato_problem* h, GridBox* box);
+
+}  // namespace plato

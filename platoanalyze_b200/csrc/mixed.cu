@@ -24,6 +24,7 @@
 
 #include <cuda_fp16.h>
 
+#include "fcg_grid.cuh"
 #include "plato_internal.cuh"
 #include "solver_common.cuh"
 
@@ -56,12 +57,6 @@ constexpr int kMaxRestarts = 8;  // restarts from the true residual (see the pla
 
 enum InnerKind { INNER_SELL64 = 0, INNER_SELL32 = 1, INNER_SELL16 = 2, INNER_EBE32 = 3, INNER_EBE64 = 4,
                  INNER_SELL16S = 5 };
-
-struct ChebCoef {
-    float c0;      // first step: d = c0 Dinv r
-    float c1[64];  // step k: d_k = c1[k] d_(k-1) + c2[k] Dinv res
-    float c2[64];
-};
 
 // ---- outer operator: q = A p, then p.q -> alpha = (p.r)/(p.q) ------------------------------
 
@@ -1350,9 +1345,19 @@ int fcg_poly(plato_problem* h, const double* b, double* x, plato_solve_stats* st
             if (!ev[e]) PLATO_CUDA(h, cudaEventCreateWithFlags(&ev[e], cudaEventDisableTiming));
         ChunkPlanner plan;
         plan.full = kChunk;
-        int32_t chunk = kChunk;
+        // systems that fit run their iterations in cooperative launches, hundreds in one, whatever
+        // sweep_steps says (every step of every sweep is in the launch)
+        const bool grid = !mf && !h->wave_stall && fcg_grid_ok(h);
+        int32_t chunk = grid ? 1 : kChunk;
         for (;;) {
             for (int k = 0; k < chunk; ++k, ++enqueued) {
+                if (grid) {
+                    const int bytes = kind == INNER_SELL64 ? 8 : (kind == INNER_SELL32 ? 4 : 2);
+                    rc = fcg_grid_iterations(h, bytes, scaled, inner_vals(h, kind), cc, degree, coarse ? 1 : 0, x,
+                                             res_scale, max_it);
+                    if (rc) return rc;
+                    continue;
+                }
                 const bool timed = h->timing && (enqueued % kTimingStride) == 0;
                 cudaEvent_t e0 = nullptr, e1 = nullptr;
                 if (timed) {
@@ -1393,7 +1398,7 @@ int fcg_poly(plato_problem* h, const double* b, double* x, plato_solve_stats* st
             if (have_prev) {
                 PLATO_CUDA(h, cudaEventSynchronize(ev[cur ^ 1]));
                 if (slots[cur ^ 1].done) break;
-                chunk = plan.next(slots[cur ^ 1], queued);
+                if (!grid) chunk = plan.next(slots[cur ^ 1], queued);
             }
             have_prev = true;
             cur ^= 1;
@@ -1401,6 +1406,19 @@ int fcg_poly(plato_problem* h, const double* b, double* x, plato_solve_stats* st
         PLATO_CUDA(h, cudaStreamSynchronize(s));
         PcgScalars fin;
         PLATO_CUDA(h, cudaMemcpy(&fin, h->scal, sizeof(PcgScalars), cudaMemcpyDeviceToHost));
+        if (grid) {
+            int gave_up = 0;
+            rc = fcg_grid_gave_up(h, &gave_up);
+            if (rc) return rc;
+            if (gave_up) {  // start again from this x, one launch per stage from here on
+                h->grid_off = 1;
+                fin.done = 0;
+                fin.ticket = 0u;
+                PLATO_CUDA(h, cudaMemcpyAsync(h->scal, &fin, sizeof(PcgScalars), cudaMemcpyHostToDevice, s));
+                keep_bb = true;
+                continue;
+            }
+        }
         if (wave_S > 0) {
             WaveCtl ctl{};
             PLATO_CUDA(h, cudaMemcpy(&ctl, h->wave_ctl, sizeof(WaveCtl), cudaMemcpyDeviceToHost));

@@ -1,0 +1,297 @@
+// The Jacobi-PCG iterations of systems that fit on the chip, in one cooperative launch.
+//
+// A system of a few thousand to some hundred thousand rows leaves a kernel of the launch-per-stage
+// loop (solver.cu) idle most of the time: its launch, its last-block reduction and the gap to
+// the next one cost far more than the arithmetic (20x10x10 cantilever, 455 iterations: 31.5 us
+// an iteration for three kernels over a 2.4 MB matrix).  Here one CTA per SM owns a run of SELL
+// slices for the whole solve: its part of the matrix stays in shared memory when it fits (else it
+// is read from L2), its rows' x, r, p, A p and inverse diagonal stay in registers, and an
+// iteration is
+//   A p with p = z + beta p formed at each gathered column   -> sum p.Ap over the grid -> alpha
+//   x += alpha p, r -= alpha A p, z = Dinv r                 -> sums r.z, r.r          -> beta
+// so two grid-wide sums per iteration, which are also its two barriers.  Only z and p leave the SM.
+// Bound by the two sums (1.5 to 3 us each).  Solve of a cantilever with a random density, launch per stage
+// against this: 20x10x10 15.1 -> 3.2 ms, 30x16x16 24.9 -> 5.2, 40x20x20 30.4 -> 7.5, 60x30x30 54.4 -> 20.6,
+// 64x32x32 84.5 -> 26.4.  Density filter (one unknown per row): 20x10x10 0.66 -> 0.26 ms, 80x40x40
+// 1.92 -> 0.96, 100x50x50 3.30 -> 1.69, 112x53x52 (the largest that qualifies) 4.00 -> 3.81: there the
+// CTAs read the matrix from L2 with two slices per warp, hence the limits in pcg_grid_ok.
+#include <algorithm>
+
+#include "grid.cuh"
+#include "plato_internal.cuh"
+
+namespace plato {
+
+int ensure_smem_attribute(plato_problem* h, const void* kernel, int bytes);
+SellView sell_view(const plato_problem* h);
+
+namespace {
+
+constexpr int kLaunchIters = 2048;         // iterations per launch: some ten milliseconds
+static_assert(kLaunchIters % 2 == 0, "the direction buffers swap once per iteration");
+
+struct GridPcg {
+    SellView      A;
+    int32_t       nslices;
+    int32_t       ks;        // warps per slice group
+    const double* vals;
+    const double* dinv;
+    double*       x;
+    double*       r;
+    double*       z;
+    double*       p[2];
+    int32_t       pcur;      // buffer that holds the current direction
+    int32_t       max_it;
+    int32_t       smem_bytes;
+    GridBox       box;
+    PcgScalars*   S;
+};
+
+// NB unknowns per row (3: block SELL, 1: scalar SELL), T slices per group of ks warps.
+template <int NB, int T, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1) k_pcg_grid(GridPcg a) {
+    extern __shared__ __align__(16) unsigned char grid_smem[];
+    __shared__ double sh_cta[2][32], sh_grid[2][32];
+    __shared__ double part[NB][THREADS];
+    constexpr int NE = NB * NB;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int s0 = int((int64_t)a.nslices * blockIdx.x / gridDim.x), s1 = int((int64_t)a.nslices * (blockIdx.x + 1) / gridDim.x);
+    const int kg = warp % a.ks, group = warp / a.ks, groups = (THREADS / 32) / a.ks;
+    const bool leader = kg == 0;
+
+    // this CTA's slots in shared memory, when they fit
+    const int64_t first = a.A.ptr[s0], slots = a.A.ptr[s1] - first;
+    const double* vals = a.vals + NE * first;
+    const int32_t* cols = a.A.cols + first;
+    if (slots * (8 * NE + 4) <= a.smem_bytes) {
+        double* sv = reinterpret_cast<double*>(grid_smem);
+        int32_t* sc = reinterpret_cast<int32_t*>(sv + NE * slots);
+        for (int64_t i = tid; i < NE * slots; i += THREADS) sv[i] = __ldg(vals + i);
+        for (int64_t i = tid; i < slots; i += THREADS) sc[i] = __ldg(cols + i);
+        vals = sv;
+        cols = sc;
+    }
+
+    double x[T][NB], r[T][NB], p[T][NB], ap[T][NB], di[T][NB];
+    int32_t width[T];
+    int32_t base[T];
+#pragma unroll
+    for (int t = 0; t < T; ++t) {
+        const int s = s0 + group + t * groups;
+        const int64_t row = 32 * int64_t(s) + lane;
+        width[t] = s < s1 ? a.A.width[s] : 0;
+        base[t] = s < s1 ? int32_t(a.A.ptr[s] - first) : 0;
+        const bool own = leader && s < s1 && row < a.A.num_rows;
+#pragma unroll
+        for (int d = 0; d < NB; ++d) {
+            x[t][d] = own ? a.x[NB * row + d] : 0.0;
+            r[t][d] = own ? a.r[NB * row + d] : 0.0;
+            p[t][d] = own ? a.p[a.pcur][NB * row + d] : 0.0;
+            di[t][d] = own ? a.dinv[NB * row + d] : 0.0;
+        }
+    }
+    double rz = a.S->rz, rr = a.S->rr, beta = a.S->beta, pap = 0.0, alpha = 0.0;
+    const double tol2 = a.S->tol2;
+    int32_t iter = a.S->iter, done = a.S->done, nonfinite = a.S->nonfinite;
+    uint32_t epoch = 0;  // barriers of this launch
+    int pcur = a.pcur;
+    __syncthreads();
+
+    for (int it = 0; it < kLaunchIters && !done; ++it) {
+        const double* pold = a.p[pcur];
+        double* pnew = a.p[pcur ^ 1];
+        double s2[2] = {0.0, 0.0};
+#pragma unroll
+        for (int t = 0; t < T; ++t) {
+            const int s = s0 + group + t * groups;
+            double acc[NB];
+#pragma unroll
+            for (int d = 0; d < NB; ++d) acc[d] = 0.0;
+            const int32_t* c0 = cols + base[t] + lane;
+            const double* v0 = vals + NE * base[t] + lane;
+#pragma unroll 4
+            for (int k = kg; k < width[t]; k += a.ks) {
+                const int64_t c = c0[32 * k];
+                double pc[NB];
+#pragma unroll
+                for (int d = 0; d < NB; ++d) pc[d] = a.z[NB * c + d] + beta * pold[NB * c + d];
+#pragma unroll
+                for (int i = 0; i < NB; ++i)
+#pragma unroll
+                    for (int j = 0; j < NB; ++j) acc[i] += v0[32 * (NE * k + NB * i + j)] * pc[j];
+            }
+            if (a.ks > 1) {
+                if (t > 0) __syncthreads();  // the leaders have read the slice before
+#pragma unroll
+                for (int d = 0; d < NB; ++d) part[d][tid] = acc[d];
+                __syncthreads();
+                if (leader)
+#pragma unroll
+                    for (int d = 0; d < NB; ++d)
+                        for (int q = 1; q < a.ks; ++q) acc[d] += part[d][tid + 32 * q];
+            }
+            const int64_t row = 32 * int64_t(s) + lane;
+            if (leader && s < s1 && row < a.A.num_rows) {
+#pragma unroll
+                for (int d = 0; d < NB; ++d) {
+                    p[t][d] = di[t][d] * r[t][d] + beta * p[t][d];
+                    pnew[NB * row + d] = p[t][d];
+                    ap[t][d] = acc[d];
+                    s2[0] += p[t][d] * acc[d];
+                }
+            }
+        }
+        pcur ^= 1;
+        double s1v[1] = {s2[0]};
+        if (!grid_sum<1>(s1v, a.box, ++epoch, sh_cta, sh_grid)) break;
+        pap = s1v[0];
+        alpha = rz / pap;
+        if (!isfinite(alpha) || pap <= 0.0) {
+            nonfinite = 1;
+            done = 1;
+            break;
+        }
+        s2[0] = s2[1] = 0.0;
+#pragma unroll
+        for (int t = 0; t < T; ++t) {
+            const int s = s0 + group + t * groups;
+            const int64_t row = 32 * int64_t(s) + lane;
+            if (leader && s < s1 && row < a.A.num_rows) {
+#pragma unroll
+                for (int d = 0; d < NB; ++d) {
+                    x[t][d] += alpha * p[t][d];
+                    r[t][d] -= alpha * ap[t][d];
+                    const double zi = di[t][d] * r[t][d];
+                    a.z[NB * row + d] = zi;
+                    s2[0] += r[t][d] * zi;
+                    s2[1] += r[t][d] * r[t][d];
+                }
+            }
+        }
+        if (!grid_sum<2>(s2, a.box, ++epoch, sh_cta, sh_grid)) break;
+        beta = s2[0] / rz;
+        rz = s2[0];
+        rr = s2[1];
+        ++iter;
+        if (!isfinite(rz) || !isfinite(rr)) nonfinite = 1;
+        if (nonfinite || rr <= tol2 || iter >= a.max_it) done = 1;
+    }
+#pragma unroll
+    for (int t = 0; t < T; ++t) {
+        const int s = s0 + group + t * groups;
+        const int64_t row = 32 * int64_t(s) + lane;
+        if (leader && s < s1 && row < a.A.num_rows)
+#pragma unroll
+            for (int d = 0; d < NB; ++d) {
+                a.x[NB * row + d] = x[t][d];
+                a.r[NB * row + d] = r[t][d];
+            }
+    }
+    if (blockIdx.x == 0 && tid == 0) {
+        a.S->rz = rz;
+        a.S->rz_new = rz;
+        a.S->rr = rr;
+        a.S->pAp = pap;
+        a.S->alpha = alpha;
+        a.S->beta = beta;
+        a.S->iter = iter;
+        a.S->nonfinite = nonfinite;
+        a.S->done = done;
+    }
+}
+
+template <int NB>
+constexpr int grid_threads() { return NB == 3 ? 512 : 1024; }
+
+template <int NB, int T>
+int launch_grid(plato_problem* h, GridPcg& a, int grid) {
+    constexpr int THREADS = grid_threads<NB>();
+    const void* kernel = reinterpret_cast<const void*>(k_pcg_grid<NB, T, THREADS>);
+    PLATO_RC(ensure_smem_attribute(h, kernel, a.smem_bytes));
+    PLATO_CUDA(h, launch_cooperative(k_pcg_grid<NB, T, THREADS>, grid, THREADS, size_t(a.smem_bytes), h->stream, a));
+    PLATO_LAUNCH_CHECK(h);
+    return PLATO_OK;
+}
+
+}  // namespace
+
+int grid_box(plato_problem* h, GridBox* box) {
+    int sms = 0;
+    PLATO_CUDA(h, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
+    const size_t bytes = sizeof(double) * 2 * kGridValues * size_t(sms);
+    if (!h->grid_box) {
+        PLATO_CUDA(h, cudaMalloc(&h->grid_box, bytes + 128));
+        PLATO_CUDA(h, cudaMemsetAsync(h->grid_box, 0, bytes + 128, h->stream));
+    }
+    box->count = static_cast<uint32_t*>(h->grid_box);  // a cache line of its own
+    box->abort = reinterpret_cast<int32_t*>(static_cast<char*>(h->grid_box) + 64);
+    box->box = reinterpret_cast<double*>(static_cast<char*>(h->grid_box) + 128);
+    PLATO_CUDA(h, cudaMemsetAsync(box->count, 0, sizeof(uint32_t), h->stream));
+    return PLATO_OK;
+}
+
+// Whether the iterations of this system run in cooperative launches: every slice has a group of
+// warps (one slice a group for block systems, at most two for scalar ones), nothing else wants a
+// look between iterations (sampled timings, a deflated direction), and no earlier launch gave up.
+bool pcg_grid_ok(const plato_problem* h, int nb) {
+    if (h->grid_off || h->timing || h->ritz_deflating) return false;
+    const int64_t warps = (nb == 3 ? grid_threads<3>() : grid_threads<1>()) / 32;
+    return h->sell.nslices <= int64_t(kNumSMs) * warps * (nb == 3 ? 1 : 2);
+}
+
+// Runs the iterations from the state that k_pcg_start left (r, z, p = z, the scalars) until the scalars
+// say done; *gave_up is set when a launch gave up.  p2 is the second direction buffer.
+int pcg_grid(plato_problem* h, int nb, const double* vals, const double* dinv, double* x, double* p2, int32_t max_it,
+             PcgScalars* fin, int* gave_up) {
+    *gave_up = 0;
+    int sms = 0, coop = 0;
+    PLATO_CUDA(h, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
+    PLATO_CUDA(h, cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h->device));
+    const int warps = (nb == 3 ? grid_threads<3>() : grid_threads<1>()) / 32;
+    const int grid = std::min({sms, h->sell.nslices, 32 * warps});
+    const int per_cta = (h->sell.nslices + grid - 1) / grid;
+    if (!coop || per_cta > 2 * warps || (nb == 3 && per_cta > warps)) {
+        PLATO_CUDA(h, cudaMemcpyAsync(h->scal_host, h->scal, sizeof(PcgScalars), cudaMemcpyDeviceToHost, h->stream));
+        PLATO_CUDA(h, cudaStreamSynchronize(h->stream));
+        *fin = h->scal_host[0];
+        *gave_up = 1;
+        return PLATO_OK;
+    }
+    GridPcg a{};
+    a.A = sell_view(h);
+    a.nslices = h->sell.nslices;
+    a.ks = 1;
+    while (2 * a.ks * per_cta <= warps) a.ks *= 2;
+    a.vals = vals;
+    a.dinv = dinv;
+    a.x = x;
+    a.r = h->v_r;
+    a.z = h->v_z;
+    a.p[0] = h->v_p;
+    a.p[1] = p2;
+    a.max_it = max_it;
+    a.S = h->scal;
+    // shared memory for the average CTA's slots and a tenth more; a CTA with more reads L2
+    const int64_t want = (h->sell.total_slots / grid + 32) * (8 * nb * nb + 4) * 11 / 10;
+    a.smem_bytes = want <= kGridSmemMax - (nb == 3 ? 512 * 24 : 1024 * 8) - 2048 ? int((want + 15) / 16 * 16) : 0;
+    for (;;) {
+        PLATO_RC(grid_box(h, &a.box));
+        if (nb == 3) PLATO_RC((launch_grid<3, 1>(h, a, grid)));
+        else if (per_cta <= warps) PLATO_RC((launch_grid<1, 1>(h, a, grid)));
+        else PLATO_RC((launch_grid<1, 2>(h, a, grid)));
+        int32_t abort = 0;
+        PLATO_CUDA(h, cudaMemcpyAsync(h->scal_host, h->scal, sizeof(PcgScalars), cudaMemcpyDeviceToHost, h->stream));
+        PLATO_CUDA(h, cudaMemcpyAsync(&abort, a.box.abort, sizeof(abort), cudaMemcpyDeviceToHost, h->stream));
+        PLATO_CUDA(h, cudaStreamSynchronize(h->stream));
+        *fin = h->scal_host[0];
+        if (abort) {
+            PLATO_CUDA(h, cudaMemsetAsync(a.box.abort, 0, sizeof(abort), h->stream));
+            *gave_up = 1;
+            return PLATO_OK;
+        }
+        if (fin->done) return PLATO_OK;
+        // after an even number of iterations the current direction is in the same buffer again
+    }
+}
+
+}  // namespace plato

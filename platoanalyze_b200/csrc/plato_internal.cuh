@@ -250,6 +250,8 @@ struct plato_problem {
     int32_t partials_len = 0;
     PcgScalars* scal = nullptr;    // device
     PcgScalars* scal_host = nullptr;  // pinned mirror
+    void*    grid_box = nullptr;   // counter, abort flag and boxes of the cooperative Krylov loops (grid.cuh)
+    int      grid_off = 0;         // one of its waits ran out on this handle: one launch per stage from then on
     double* red_out = nullptr;     // device scalar result of a reduction
     uint32_t* red_ticket = nullptr;
     // mixed-precision and matrix-free work (allocated on first use)

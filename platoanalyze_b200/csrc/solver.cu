@@ -23,6 +23,9 @@ int launch_crs_to_sell(plato_problem* h, const double* crs, double* out64, float
                        double* dinv, float* dinv32);
 int launch_assemble_sell(plato_problem* h, const double* z, double* v64, float* v32, void* v16, double* dinv,
                          float* dinv32);
+bool pcg_grid_ok(const plato_problem* h, int nb);
+int pcg_grid(plato_problem* h, int nb, const double* vals, const double* dinv, double* x, double* p2, int32_t max_it,
+             PcgScalars* fin, int* gave_up);
 
 namespace {
 
@@ -299,14 +302,15 @@ int prepare_operator(plato_problem* h, const double* crs, const double* z) {
     return launch_crs_to_sell(h, crs, h->sell64, nullptr, nullptr, h->v_dinv, nullptr);
 }
 
-// Jacobi-PCG on n unknowns with the operator apply(in, out, S) (S != nullptr: fused p.Ap and
-// alpha) and inverse diagonal dinv; x holds the initial guess on entry.  With p2 (n values)
+// Jacobi-PCG on n unknowns (nb per row of the SELL matrix `vals`) with the operator apply(in, out, S)
+// (S != nullptr: fused p.Ap and alpha) and inverse diagonal dinv; x holds the initial guess on entry.
+// A system that fits runs its iterations in cooperative launches (pcg_grid.cu).  With p2 (n values)
 // the search direction is formed inside the operator instead of by its own kernel:
 // apply_dir(p_old, p_new, Ap, S) computes p_new = z + beta p_old and Ap = A p_new, and the
 // two direction buffers alternate.
 template <class Apply, class ApplyDir>
-static int pcg_run(plato_problem* h, int64_t n, Apply apply, ApplyDir apply_dir, double* p2, const double* dinv,
-                   const double* b, double* x, plato_solve_stats* stats) {
+static int pcg_run(plato_problem* h, int64_t n, int nb, const double* vals, Apply apply, ApplyDir apply_dir, double* p2,
+                   const double* dinv, const double* b, double* x, plato_solve_stats* stats) {
     cudaStream_t s = h->stream;
     const double tol = h->opts.tolerance;
     const int32_t max_it = h->opts.max_iterations;
@@ -345,7 +349,23 @@ static int pcg_run(plato_problem* h, int64_t n, Apply apply, ApplyDir apply_dir,
         ChunkPlanner plan;
         plan.full = kChunk;
         int32_t chunk = kChunk;
-        for (;;) {
+        PcgScalars fin;
+        const bool grid = pcg_grid_ok(h, nb);
+        if (grid) {  // the whole loop in cooperative launches
+            int gave_up = 0;
+            rc = pcg_grid(h, nb, vals, dinv, x, p2 ? p2 : h->v_tmp, max_it, &fin, &gave_up);
+            if (rc) return rc;
+            if (gave_up) {  // start again from this x, one launch per stage from here on
+                h->grid_off = 1;
+                PcgScalars cont = fin;
+                cont.done = 0;
+                cont.ticket = 0u;
+                PLATO_CUDA(h, cudaMemcpyAsync(h->scal, &cont, sizeof(PcgScalars), cudaMemcpyHostToDevice, s));
+                keep_bb = true;
+                continue;
+            }
+        }
+        while (!grid) {
             for (int k = 0; k < chunk; ++k, ++enqueued) {
                 const bool timed = h->timing && (enqueued % kTimingStride) == 0;
                 cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -385,9 +405,10 @@ static int pcg_run(plato_problem* h, int64_t n, Apply apply, ApplyDir apply_dir,
             have_prev = true;
             cur ^= 1;
         }
-        PLATO_CUDA(h, cudaStreamSynchronize(s));
-        PcgScalars fin;
-        PLATO_CUDA(h, cudaMemcpy(&fin, h->scal, sizeof(PcgScalars), cudaMemcpyDeviceToHost));
+        if (!grid) {
+            PLATO_CUDA(h, cudaStreamSynchronize(s));
+            PLATO_CUDA(h, cudaMemcpy(&fin, h->scal, sizeof(PcgScalars), cudaMemcpyDeviceToHost));
+        }
         rc = collect_timing(h, timed_iters, fin.iter - iter_base);
         if (rc) return rc;
         iter_base = fin.iter;
@@ -444,7 +465,7 @@ int pcg_fp64(plato_problem* h, const double* b, double* x, plato_solve_stats* st
         return PLATO_OK;
     };
     auto no_dir = [](const double*, double*, double*, PcgScalars*) -> int { return PLATO_OK; };
-    return pcg_run(h, 3 * (int64_t)h->N, apply, no_dir, nullptr, h->v_dinv, b, x, stats);
+    return pcg_run(h, 3 * (int64_t)h->N, 3, A, apply, no_dir, nullptr, h->v_dinv, b, x, stats);
 }
 
 // Scalar Jacobi-PCG (one unknown per node) on SELL values `vals` with inverse diagonal dinv;
@@ -466,7 +487,7 @@ int pcg_scalar(plato_problem* h, const double* vals, const double* dinv, const d
         PLATO_LAUNCH_CHECK(h);
         return PLATO_OK;
     };
-    return pcg_run(h, (int64_t)h->N, apply, apply_dir, h->v_tmp, dinv, b, x, stats);
+    return pcg_run(h, (int64_t)h->N, 1, vals, apply, apply_dir, h->v_tmp, dinv, b, x, stats);
 }
 
 // y = A x for a scalar SELL matrix.
