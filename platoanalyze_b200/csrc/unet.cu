@@ -8,11 +8,12 @@
 // parameters FP32 (Adam) with BF16 copies for the tensor cores.
 //
 //  * Convolution (forward and data gradient): implicit GEMM, M = voxels, N = output
-//    channels, K = taps x input channels, mma.sync.m16n8k16 BF16 -> FP32; each warp owns
-//    32 voxels x all output channels; A fragments are gathered straight from the haloed
-//    tensor (pairs of channels are 32-bit words), B fragments from the weights laid out
-//    [tap][out][in].  Bias, ReLU and FP32 accumulation are fused in the epilogue.  The data
-//    gradient is the same convolution with flipped, transposed weights.
+//    channels, K = taps x input channels, on tcgen05 with FP32 accumulators in tensor memory:
+//    k_conv_tz marches along z and uses each input plane for three output planes, k_conv_tc
+//    takes the layers whose weights it cannot keep beside its slabs (96 -> 32, 64 -> 64), those of
+//    more than 80 output channels and the 1x1x1 head.  k_conv (mma.sync, A fragments gathered from the haloed
+//    tensor) is the second family of the API.  Bias, ReLU and FP32 accumulation are fused in
+//    the epilogue.  The data gradient is the same convolution with flipped, transposed weights.
 //  * Weight gradient: GEMM over voxels, M = output channels, N = input channels, K =
 //    voxels; a CTA stages 64-voxel tiles of the masked output gradient and of the shifted
 //    input in shared memory and feeds the tensor cores with ldmatrix.trans; partial sums
@@ -541,6 +542,287 @@ k_conv_tc(TView in, const bf16* __restrict__ Wt, const float* __restrict__ bias,
     __syncthreads();
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * ACC_COLS) : "memory");
+}
+
+// ---- convolution, marching along z ---------------------------------------------------------
+// The 3x3x3 convolution of k_conv_tc with each input plane used for the three output planes it
+// reaches at once.  A CTA's item is a column of 128 consecutive positions of a (y, x) plane and a
+// run of output planes z; it walks the input planes in order.  For input plane zi the 9 (dy, dx)
+// taps' A windows (the same slab, the same descriptors as k_conv_tc) are multiplied with the
+// weights of all three dz side by side: N = 3 COUTP, columns of output planes zi - 1, zi, zi + 1, which
+// lie next to one another in tensor memory (a ring of R accumulators; where the ring wraps, or
+// at the ends of a run, the MMA is issued in pieces of one or two planes).  With few output
+// channels an MMA costs what reading its A window costs (128 x 16 x 16: about 50 cycles, against 8
+// of arithmetic), so one window for three planes is a third of that cost, and a plane's slab is
+// copied once instead of three times.  An output plane is complete after plane zi + 1; its
+// accumulator is then read, zeroed for the next round of the ring (tcgen05.st) and stored, while the
+// next plane's MMAs run.  The sum of an output element runs over dz, dy, dx and channel chunks in
+// the same order as in k_conv_tc.  Bound by the A windows' reads; batch 8 on 68x36x36, against k_conv_tc:
+// 16 -> 16 channels 86 -> 51 us, 48 -> 16 246 -> 120 us (training step 2.91 -> 2.57 ms).
+__device__ __forceinline__ void tmem_zero16(uint32_t taddr) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr),
+        "r"(0)
+        : "memory");
+}
+
+// accumulators in the ring: at least 4 (see the loop), more where tensor memory leaves room, since
+// two of R planes wrap
+template <int COUTP>
+constexpr int tz_ring() {
+    return COUTP <= 32 ? 8 : (COUTP == 48 ? 5 : 4);
+}
+template <int COUTP>
+constexpr int tz_tmem_cols() {
+    return tz_ring<COUTP>() * COUTP <= 128 ? 128 : 256;
+}
+
+struct TzGeom {
+    int32_t  ncol;    // columns of 128 positions per plane
+    int32_t  nseg;    // runs of output planes per column
+    int32_t  seglen;  // output planes per run (the last may be shorter)
+    int32_t  nitems;  // batch * ncol * nseg
+    int32_t  ptotal;  // positions of the haloed tensor
+    int32_t  rows, nbuf, lag;
+    uint32_t w_bytes, buf_bytes;
+};
+
+// Position in a CTA's sequence of planes: item k of this CTA, input plane z (haloed index).
+struct TzCursor {
+    int     item, z, z_last;      // current input plane and the run's last one
+    int     za, zb;               // output planes [za, zb)
+    int32_t base;                 // in-plane position of the tile's row 0, plus the batch item's first position
+    int     out0;                 // running number of output plane za
+};
+
+template <int CIN, int COUT, bool RELU, bool OUT_F32, bool ACCUM>
+__global__ void __launch_bounds__(128)
+k_conv_tz(TView in, const bf16* __restrict__ Wt, const float* __restrict__ bias, TView out, TzGeom g,
+          int* __restrict__ err) {
+    constexpr int COUTP = (COUT + 15) / 16 * 16;
+    static_assert(CIN % 16 == 0 && COUT % 16 == 0 && 3 * COUTP <= 256, "UMMA shape");
+    constexpr bool SW = CIN == 16;  // 16-channel slabs: rows of 32 B in the 32-byte swizzle
+    constexpr int R = tz_ring<COUTP>();
+    constexpr uint32_t BTAP = 3u * COUTP * CIN * 2;           // one (dy, dx) tap: the weights of three dz
+    constexpr uint32_t LBO_B = 3u * (COUTP / 8) * 128;
+    const uint32_t LBO_A = uint32_t(g.rows) * 16u;
+    extern __shared__ __align__(128) uint8_t tc_smem[];
+    __shared__ __align__(8) uint64_t bar[5];  // MMA completion per slab buffer (4), all MMAs (1)
+    __shared__ uint32_t tmem_slot;
+    __shared__ float sbias[COUTP];
+    const int tid = threadIdx.x, warp = tid >> 5;
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
+                     "r"(tz_tmem_cols<COUTP>())
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (tid == 0) {
+        for (int q = 0; q < 5; ++q) mbar_init(&bar[q], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    for (int c = tid; c < COUTP; c += 128) sbias[c] = bias ? bias[c] : 0.f;
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_slot;
+    const uint32_t my_lanes = tmem + (uint32_t(32 * warp) << 16);
+#pragma unroll
+    for (int c = 0; c < R * COUTP; c += 16) tmem_zero16(my_lanes + uint32_t(c));
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");  // the first MMAs follow a barrier
+
+    const int D = in.D;
+    const int32_t sy = in.W + 2, sz = (in.H + 2) * sy;
+    const int halo = sy + 1, nrows = kTcRows + 2 * halo;
+    const int nbuf = g.nbuf, lag = g.lag;
+    const bf16* __restrict__ ip = static_cast<const bf16*>(in.p);
+    const uint32_t wbase = smem_u32(tc_smem), bbase = wbase + g.w_bytes;
+
+    // the runs of this CTA, one after the other: item blockIdx.x, + gridDim.x, ...
+    auto load_item = [&](TzCursor& c) {
+        const int seg = c.item % g.nseg, rest = c.item / g.nseg, col = rest % g.ncol, b = rest / g.ncol;
+        c.za = 1 + seg * g.seglen;
+        c.zb = min(c.za + g.seglen, D + 1);
+        c.z = max(c.za - 1, 1);
+        c.z_last = min(c.zb, D);
+        c.base = b * (D + 2) * sz + sy + 1 + col * kTcRows;
+    };
+    auto advance = [&](TzCursor& c) {
+        if (c.z < c.z_last) {
+            ++c.z;
+            return;
+        }
+        c.out0 += c.zb - c.za;
+        c.item += gridDim.x;
+        if (c.item < g.nitems) load_item(c);
+    };
+    TzCursor copy{}, issue{}, done{};
+    copy.item = blockIdx.x;
+    load_item(copy);
+    issue = done = copy;
+    int nsteps = 0;
+    for (TzCursor c = copy; c.item < g.nitems;) {
+        nsteps += c.z_last - c.z + 1;
+        c.z = c.z_last;
+        advance(c);
+    }
+
+    // bias, ReLU and store of the output planes that are complete after input plane c.z; thread t owns
+    // TMEM lane t = the column's row t
+    auto epilogue = [&](const TzCursor& c) {
+        const int first = max(c.za, c.z - 1), last = c.z == D ? c.zb - 1 : c.z - 1;
+        for (int zo = first; zo <= last; ++zo) {
+            const uint32_t acc = my_lanes + uint32_t(((c.out0 + zo - c.za) % R) * COUTP);
+            const int32_t p = c.base + zo * sz + tid;
+            const uint32_t q = uint32_t(c.base + tid) % uint32_t(sz);  // in-plane position: base is (b (D + 2)) sz + it
+            const uint32_t y = q / uint32_t(sy), x = q - y * uint32_t(sy);
+            const bool row_ok = x >= 1u && x <= uint32_t(in.W) && y >= 1u && y <= uint32_t(in.H) &&
+                                uint32_t(c.base + tid) - q == uint32_t(c.base) - uint32_t(c.base) % uint32_t(sz);
+            const int64_t obase = int64_t(p) * out.ld + out.c0;
+#pragma unroll
+            for (int c0 = 0; c0 < COUTP; c0 += 16) {
+                uint32_t r[16];
+                tmem_ld16(acc + uint32_t(c0), r);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                tmem_zero16(acc + uint32_t(c0));
+                if (!row_ok) continue;
+                float v[16];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    v[j] = __uint_as_float(r[j]) + sbias[c0 + j];
+                    if (RELU) v[j] = fmaxf(v[j], 0.f);
+                }
+                if (OUT_F32) {
+                    float* op = static_cast<float*>(out.p) + obase + c0;
+#pragma unroll
+                    for (int j = 0; j < 16; j += 4) {
+                        float4 w4 = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                        if (ACCUM) {
+                            const float4 o4 = *reinterpret_cast<const float4*>(op + j);
+                            w4.x += o4.x; w4.y += o4.y; w4.z += o4.z; w4.w += o4.w;
+                        }
+                        *reinterpret_cast<float4*>(op + j) = w4;
+                    }
+                } else {
+                    bf16* op = static_cast<bf16*>(out.p) + obase + c0;
+                    uint4 lo, hi;
+                    lo.x = pack_bf16(v[0], v[1]); lo.y = pack_bf16(v[2], v[3]);
+                    lo.z = pack_bf16(v[4], v[5]); lo.w = pack_bf16(v[6], v[7]);
+                    hi.x = pack_bf16(v[8], v[9]); hi.y = pack_bf16(v[10], v[11]);
+                    hi.z = pack_bf16(v[12], v[13]); hi.w = pack_bf16(v[14], v[15]);
+                    reinterpret_cast<uint4*>(op)[0] = lo;
+                    reinterpret_cast<uint4*>(op)[1] = hi;
+                }
+            }
+        }
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");  // the accumulator is used again after a barrier
+    };
+
+    bool ok = true;
+    int issued = 0;
+    // iteration i copies the slab of step i into buffer i % nbuf and issues the MMAs of step i - lag; then
+    // the planes that step i - lag - 1 completed are stored.  The highest accumulator that a step adds to
+    // was last used R planes before: R >= 4 keeps it clear of the planes not yet stored (those of the step
+    // before, and, at the end of a run, one more).
+    for (int i = 0; i < nsteps + lag; ++i) {
+        if (i < nsteps) {
+            const int b = i % nbuf;
+            if (i >= nbuf) {
+                bool w = true;
+                if (tid == 0) w = mbar_wait(&bar[b], uint32_t((i - nbuf) / nbuf) & 1u);
+                ok = __syncthreads_and(w) != 0;
+                if (!ok) break;
+            }
+            const uint32_t a_s = bbase + uint32_t(b) * g.buf_bytes;
+            const int32_t r0 = copy.base + copy.z * sz - halo;
+            for (int q = tid; q < nrows * (CIN / 8); q += 128) {
+                const int r = q / (CIN / 8), c8 = q - r * (CIN / 8);
+                const int32_t pos = r0 + r;
+                const bool inside = pos >= 0 && pos < g.ptotal;
+                uint32_t dst = a_s + uint32_t(c8) * LBO_A + uint32_t(r) * 16u;
+                if (SW) {
+                    const uint32_t row = a_s + 32u * uint32_t(r);
+                    dst = row + 16u * (uint32_t(c8) ^ ((row >> 7) & 1u));
+                }
+                cp_async16(dst, inside ? ip + int64_t(pos) * in.ld + in.c0 + 8 * c8 : ip, inside ? 16u : 0u);
+            }
+            if (i == 0) {  // all weights: tap (dy, dx), then rows dz = +1, 0, -1 (output planes zi - 1, zi, zi + 1)
+                for (int q = tid; q < 27 * COUTP * (CIN / 8); q += 128) {
+                    const int j = q / (3 * COUTP * (CIN / 8)), rem = q - j * (3 * COUTP * (CIN / 8));
+                    const int n = rem / (CIN / 8), c8 = rem - n * (CIN / 8);
+                    const int dz = 2 - n / COUTP, co = n % COUTP;
+                    cp_async16(wbase + uint32_t(j) * BTAP + uint32_t(c8) * LBO_B + uint32_t(n >> 3) * 128u + uint32_t(n & 7) * 16u,
+                               Wt + (int64_t(9 * dz + j) * COUTP + co) * CIN + 8 * c8, 16u);
+                }
+            }
+            advance(copy);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (i >= lag) {
+            const int s = i - lag, b = s % nbuf;
+            if (lag == 1) asm volatile("cp.async.wait_group 0;" ::: "memory");
+            else if (lag == 2) asm volatile("cp.async.wait_group 1;" ::: "memory");
+            else asm volatile("cp.async.wait_group 2;" ::: "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncthreads();
+            if (tid == 0) {
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t a_s = bbase + uint32_t(b) * g.buf_bytes;
+                const int lo = max(issue.z - 1, issue.za), hi = min(issue.z + 1, issue.zb - 1);  // output planes
+                const int slot0 = (issue.out0 + lo - issue.za) % R;
+                const int n0 = min(hi - lo + 1, R - slot0), n1 = hi - lo + 1 - n0;  // planes before and after the wrap
+                const uint32_t j0 = uint32_t(lo - (issue.z - 1));                   // weight rows of plane lo
+                const uint32_t idesc0 = umma_idesc_bf16_f32<0>() | (uint32_t(n0 * COUTP / 8) << 17);
+                const uint32_t idesc1 = umma_idesc_bf16_f32<0>() | (uint32_t(n1 * COUTP / 8) << 17);
+#pragma unroll 1
+                for (int j = 0; j < 9; ++j) {
+                    const int dy = j / 3 - 1, dx = j % 3 - 1;
+                    const uint32_t a_t = a_s + uint32_t(halo + dy * sy + dx) * (SW ? 32u : 16u);
+                    const uint32_t w_t = wbase + uint32_t(j) * BTAP + j0 * (COUTP / 8) * 128u;
+#pragma unroll
+                    for (int kc = 0; kc < CIN / 16; ++kc) {
+                        const uint64_t da = SW ? umma_smem_desc_sw32(a_t) : umma_smem_desc(a_t + 2u * kc * LBO_A, LBO_A, 128u);
+                        umma_bf16(tmem + uint32_t(slot0 * COUTP), da, umma_smem_desc(w_t + 2u * kc * LBO_B, LBO_B, 128u), idesc0, 1u);
+                        if (n1 > 0)
+                            umma_bf16(tmem, da,
+                                      umma_smem_desc(w_t + uint32_t(n0) * (COUTP / 8) * 128u + 2u * kc * LBO_B, LBO_B, 128u),
+                                      idesc1, 1u);
+                    }
+                }
+                umma_commit(&bar[b]);
+            }
+            ++issued;
+            advance(issue);
+            if (s >= 1) {
+                bool w = true;
+                if (tid == 0) w = mbar_wait(&bar[(s - 1) % nbuf], uint32_t((s - 1) / nbuf) & 1u);
+                ok = __syncthreads_and(w) != 0;
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                epilogue(done);
+                advance(done);
+            }
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    bool fin = true;
+    if (tid == 0) {
+        if (issued > 0) umma_commit(&bar[4]);
+        fin = issued == 0 || mbar_wait(&bar[4], 0u);
+    }
+    const bool good = __syncthreads_and(ok && fin) != 0;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (good) {
+        if (nsteps > 0) epilogue(done);
+    } else if (tid == 0) {
+        atomicExch(err, 1);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tz_tmem_cols<COUTP>()) : "memory");
 }
 
 // ---- weight gradient --------------------------------------------------------------------
@@ -1196,6 +1478,54 @@ bool tc_plan(int rows, TcGeom& g, uint32_t& smem, int& ctas_per_sm) {
     return true;
 }
 
+// Shared memory, pipeline and runs of a k_conv_tz launch: all weights resident beside 2 to 4 slab
+// buffers, and the number of runs per column that lets the most loaded CTA walk the fewest planes (a
+// run reads two planes more than it writes).  False when the weights do not fit.
+template <int CIN, int COUTP>
+bool tz_plan(const TView& in, int64_t ptotal, TzGeom& g, uint32_t& smem, int& grid) {
+    constexpr uint32_t kMaxDyn = 227u * 1024u - 1280u, kSmPerSm = 228u * 1024u, kPerCtaExtra = 1024u + 1280u;
+    constexpr int tmem_ctas = 512 / tz_tmem_cols<COUTP>();
+    auto r128 = [](uint32_t v) { return (v + 127u) & ~127u; };
+    const int sy = in.W + 2, rows = tc_row_stride(kTcRows + 2 * (sy + 1), CIN / 8);
+    const uint32_t a = r128(uint32_t(rows) * CIN * 2), w = r128(27u * COUTP * CIN * 2);
+    // more CTAs than tensor memory holds must not fit: one that waits in tcgen05.alloc waits for a whole
+    // persistent CTA
+    const uint32_t guard = kSmPerSm / uint32_t(tmem_ctas + 1) - kPerCtaExtra + 128u;
+    int best = 0, occ = 0;
+    for (int nb = 2; nb <= 4; ++nb) {
+        const uint32_t need = std::max(w + uint32_t(nb) * a, guard);
+        if (need > kMaxDyn) break;
+        const int o = std::min<int>(tmem_ctas, int(kSmPerSm / (need + kPerCtaExtra)));
+        if (o * (nb - 1) > best) {
+            best = o * (nb - 1);
+            g.nbuf = nb;
+            g.lag = nb - 1;
+            smem = need;
+            occ = o;
+        }
+    }
+    if (best == 0) return false;
+    g.rows = rows;
+    g.w_bytes = w;
+    g.buf_bytes = a;
+    g.ptotal = int32_t(ptotal);
+    g.ncol = ((in.H - 1) * sy + in.W + kTcRows - 1) / kTcRows;
+    const int64_t columns = int64_t(in.B) * g.ncol, ctas = int64_t(sm_count()) * occ;
+    int64_t least = INT64_MAX;
+    for (int n = 1; n <= in.D; ++n) {
+        const int len = (in.D + n - 1) / n, runs = (in.D + len - 1) / len;
+        const int64_t planes = (columns * runs + ctas - 1) / ctas * std::min(len + 2, in.D);
+        if (planes < least) {
+            least = planes;
+            g.nseg = runs;
+            g.seglen = len;
+        }
+    }
+    g.nitems = int32_t(columns * g.nseg);
+    grid = int(std::min<int64_t>(g.nitems, ctas));
+    return true;
+}
+
 // launch helpers (dispatch on the layer's channel counts)
 template <int CIN, int COUT, int TAPS, bool RELU, bool F32, bool ACC>
 int conv_launch(cudaStream_t s, const ConvPath& P, TView in, const bf16* w, const float* b, TView out, int64_t nvox) {
@@ -1206,6 +1536,18 @@ int conv_launch(cudaStream_t s, const ConvPath& P, TView in, const bf16* w, cons
         constexpr int COUTP = (COUT + 15) / 16 * 16;
         const int64_t sy = in.W + 2, sz = int64_t(in.H + 2) * sy;
         const int64_t ptotal = int64_t(in.B) * (in.D + 2) * sz;
+        if constexpr (TAPS == 27 && COUT % 16 == 0 && 3 * COUT <= 256) {
+            TzGeom tz{};
+            uint32_t tz_smem = 0;
+            int tz_grid = 0;
+            if (ptotal < (int64_t(1) << 31) && tz_plan<CIN, COUTP>(in, ptotal, tz, tz_smem, tz_grid)) {
+                auto kernel = k_conv_tz<CIN, COUT, RELU, F32, ACC>;
+                UCUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(tz_smem)));
+                kernel<<<tz_grid, 128, tz_smem, s>>>(in, w, b, out, tz, P.err);
+                ULAUNCH();
+                return PLATO_OK;
+            }
+        }
         const int nrows = kTcRows + (TAPS == 27 ? 2 * int(sy + 1) : 0);
         TcGeom g{};
         uint32_t smem = 0;
