@@ -15,8 +15,8 @@
 //    tensor) is the second family of the API.  Bias, ReLU and FP32 accumulation are fused in
 //    the epilogue.  The data gradient is the same convolution with flipped, transposed weights.
 //  * Weight gradient: GEMM over voxels, M = output channels, N = input channels, K =
-//    voxels; a CTA stages 64-voxel tiles of the masked output gradient and of the shifted
-//    input in shared memory and feeds the tensor cores with ldmatrix.trans; partial sums
+//    voxels; a CTA stages 128-position tiles of the masked output gradient and the input slabs
+//    around them in shared memory and feeds the tensor cores with ldmatrix.trans; partial sums
 //    are added to the FP32 gradient with atomics.
 //  * 2x2x2 average pooling, nearest upsampling, the ReLU gradient mask, the loss and Adam
 //    are element-wise kernels.
@@ -838,6 +838,11 @@ k_conv_tz(TView in, const bf16* __restrict__ Wt, const float* __restrict__ bias,
 // rows of one operand at a uniform shared-memory stride; here M is 16 output channels, and the
 // taps that would fill it read the slab at non-uniform shifts.)
 constexpr int kWgRows = 128;  // positions per tile (8 k-steps)
+// Warps of a CTA, all on the same staged tile: the kernel waits for ldmatrix and the MMAs most of the
+// time, and shared memory lets three CTAs on an SM, so 8 warps each hide that better than 4, each
+// with one block of 16 output channels (one A fragment per k-step).  Batch 8 on 68x36x36, 48 -> 16 channels
+// 288 -> 163 us, 16 -> 16 79 -> 63 us; 96 -> 32 (34x18x18) 167 -> 92 us.
+constexpr int kWgWarps = 8, kWgThreads = 32 * kWgWarps;
 
 __device__ __forceinline__ void ldsm_x4_t(uint32_t (&r)[4], const bf16* p) {
     const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -856,7 +861,8 @@ template <int CIN, int COUT, int TAPS>
 constexpr int wg_groups() {
     if (TAPS == 1) return 1;
     constexpr int per_tap = (COUT / 16) * (CIN / 8);
-    return (27 * per_tap + 3) / 4 <= 18 ? 1 : (9 * per_tap + 3) / 4 <= 18 ? 3 : (3 * per_tap + 3) / 4 <= 18 ? 9 : 27;
+    constexpr int most = 18 * kWgWarps;
+    return 27 * per_tap <= most ? 1 : 9 * per_tap <= most ? 3 : 3 * per_tap <= most ? 9 : 27;
 }
 
 // offset of tap t of a 3x3x3 stencil in haloed positions
@@ -871,7 +877,7 @@ __host__ __device__ __forceinline__ int wg_halfwidth(int sy) {
 }
 
 template <int CIN, int COUT, int TAPS, int G>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(kWgThreads)
 k_conv_wgrad(TView x, TView dy, float* __restrict__ dW, int cout_real, int32_t pfirst, int32_t plast, int32_t ptotal,
              int32_t ntiles, int rows_pad, uint32_t stage_elems) {
     static_assert(COUT % 16 == 0 && CIN % 16 == 0, "channel counts");
@@ -879,10 +885,10 @@ k_conv_wgrad(TView x, TView dy, float* __restrict__ dW, int cout_real, int32_t p
     constexpr int NSL = (TAPS == 27 && G == 1) ? 3 : 1;   // x slabs per tile (one per z offset)
     constexpr int LDY = COUT + 8, LDX = CIN + 8;          // padded rows: 16-byte aligned, no ldmatrix conflicts
     constexpr int T = TPG * (COUT / 16) * (CIN / 8);      // output tiles of 16 x 8
-    // with at most two output tiles (the 1x1x1 head), pairs of warps share a tile and split its
-    // k-steps (even / odd), so all four warps work; each adds its own partial sums
-    constexpr int KSPLIT = T <= 2 ? 2 : 1;
-    constexpr int WPT = 4 / KSPLIT;
+    // with at most two output tiles (the 1x1x1 head), groups of warps share a tile and split its
+    // k-steps, so all warps work; each adds its own partial sums
+    constexpr int KSPLIT = T <= 2 ? kWgWarps / 2 : 1;
+    constexpr int WPT = kWgWarps / KSPLIT;
     constexpr int PER = (T + WPT - 1) / WPT;
     extern __shared__ __align__(16) bf16 wg_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -896,17 +902,19 @@ k_conv_wgrad(TView x, TView dy, float* __restrict__ dW, int cout_real, int32_t p
 #pragma unroll
     for (int sl = 0; sl < NSL; ++sl)
         centre[sl] = TAPS == 1 ? 0 : wg_tap_offset(NSL == 3 ? 9 * sl + 4 : g * TPG + TPG / 2, sy, sz);
-    // this warp's output tiles: element offset of its B rows (k-step 0, lane's row) and its A block
-    int boff[PER], mtile[PER];
+    // this warp's output tiles: the block of 16 output channels is the same for all of them (one A
+    // fragment per k-step); element offset of the B rows (k-step 0, lane's row)
+    constexpr int MT = COUT / 16;
+    static_assert(WPT % MT == 0, "a warp stays with its output channels");
+    const int mt = wt % MT;
+    int boff[PER];
 #pragma unroll
     for (int k = 0; k < PER; ++k) {
-        const int id = wt + WPT * k;
-        const int j = id / ((COUT / 16) * (CIN / 8)), rem = id - j * ((COUT / 16) * (CIN / 8));
-        const int mt = rem / (CIN / 8), nt = rem - mt * (CIN / 8);
+        const int id = wt + WPT * k, rest = id / MT;
+        const int j = rest / (CIN / 8), nt = rest - j * (CIN / 8);
         const int sl = NSL == 3 ? j / 9 : 0;
         const int rel = TAPS == 1 ? 0 : wg_tap_offset(g * TPG + j, sy, sz) - centre[sl];
         boff[k] = (kWgRows * LDY) + (sl * rows_pad + hw + rel + (lane & 7) + ((lane >> 3) & 1) * 8) * LDX + 8 * nt;
-        mtile[k] = mt;
     }
     float acc[PER][4];
 #pragma unroll
@@ -922,7 +930,7 @@ k_conv_wgrad(TView x, TView dy, float* __restrict__ dW, int cout_real, int32_t p
     auto stage = [&](int k, int buf) {
         const int32_t p0 = pfirst + (int(blockIdx.x) + k * int(gridDim.x)) * kWgRows;
         const uint32_t st = sbase + uint32_t(buf) * stage_elems * 2u;
-        for (int q = threadIdx.x; q < kWgRows * (COUT / 8); q += 128) {
+        for (int q = threadIdx.x; q < kWgRows * (COUT / 8); q += kWgThreads) {
             const int r = q / (COUT / 8), c8 = q - r * (COUT / 8);
             const int32_t p = p0 + r;
             bool in = p <= plast;
@@ -942,7 +950,7 @@ k_conv_wgrad(TView x, TView dy, float* __restrict__ dW, int cout_real, int32_t p
         for (int sl = 0; sl < NSL; ++sl) {
             const int32_t r0 = p0 + centre[sl] - hw;
             const uint32_t xs = st + uint32_t(kWgRows * LDY + sl * rows_pad * LDX) * 2u;
-            for (int q = threadIdx.x; q < srows * (CIN / 8); q += 128) {
+            for (int q = threadIdx.x; q < srows * (CIN / 8); q += kWgThreads) {
                 const int r = q / (CIN / 8), c8 = q - r * (CIN / 8);
                 const int32_t pos = r0 + r;
                 const bool in = pos >= 0 && pos < ptotal;
@@ -964,18 +972,16 @@ k_conv_wgrad(TView x, TView dy, float* __restrict__ dW, int cout_real, int32_t p
         for (int ks = 0; ks < kWgRows / 16; ++ks) {
             if (ks % KSPLIT != kg) continue;
             // A = dy^T (rows co, cols position): matrices (m0, k0), (m0+8, k0), (m0, k0+8), (m0+8, k0+8)
-            uint32_t a[COUT / 16][4];
+            uint32_t a[4];
             const int mat = lane >> 3, rr = lane & 7;
-#pragma unroll
-            for (int mt = 0; mt < COUT / 16; ++mt)
-                ldsm_x4_t(a[mt], sb + (16 * ks + rr + ((mat & 2) ? 8 : 0)) * LDY + 16 * mt + ((mat & 1) ? 8 : 0));
+            ldsm_x4_t(a, sb + (16 * ks + rr + ((mat & 2) ? 8 : 0)) * LDY + 16 * mt + ((mat & 1) ? 8 : 0));
 #pragma unroll
             for (int q = 0; q < PER; ++q) {
                 if (wt + WPT * q >= T) break;
                 // B = x (rows position, cols ci) at the tap's shifted slab rows
                 uint32_t b0, b1;
                 ldsm_x2_t(b0, b1, sb + boff[q] + 16 * ks * LDX);
-                mma16816(acc[q], a[mtile[q]], b0, b1);
+                mma16816(acc[q], a, b0, b1);
             }
         }
         __syncthreads();  // stage k & 1 is refilled by the next iteration's copies
@@ -986,8 +992,8 @@ k_conv_wgrad(TView x, TView dy, float* __restrict__ dW, int cout_real, int32_t p
     for (int q = 0; q < PER; ++q) {
         const int id = wt + WPT * q;
         if (id >= T) break;
-        const int j = id / ((COUT / 16) * (CIN / 8)), rem = id - j * ((COUT / 16) * (CIN / 8));
-        const int m0 = 16 * (rem / (CIN / 8)), n0 = 8 * (rem % (CIN / 8));
+        const int rest = id / MT, j = rest / (CIN / 8);
+        const int m0 = 16 * mt, n0 = 8 * (rest - j * (CIN / 8));
         float* w = dW + int64_t(g * TPG + j) * cout_real * CIN;  // rows past the real output channels are padding
         if (m0 + gq < cout_real) {
             atomicAdd(w + (m0 + gq) * CIN + n0 + 2 * tig, acc[q][0]);
@@ -1620,11 +1626,11 @@ int wgrad_launch(cudaStream_t s, TView x, TView dy, float* dW, int cout_real, in
     auto kernel = k_conv_wgrad<CIN, COUT, TAPS, G>;
     UCUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     int occ = 0;
-    UCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, 128, smem));
+    UCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kWgThreads, smem));
     const int32_t pfirst = int32_t(sz + sy + 1), plast = int32_t(halo_index(x, nvox - 1));
     const int32_t ntiles = (plast - pfirst) / kWgRows + 1;
     const int gx = int(std::max<int64_t>(1, std::min<int64_t>(ntiles, int64_t(sm_count()) * std::max(occ, 1) / G)));
-    kernel<<<dim3(unsigned(gx), unsigned(G)), 128, smem, s>>>(x, dy, dW, cout_real, pfirst, plast, int32_t(ptotal), ntiles,
+    kernel<<<dim3(unsigned(gx), unsigned(G)), kWgThreads, smem, s>>>(x, dy, dW, cout_real, pfirst, plast, int32_t(ptotal), ntiles,
                                                                rows_pad, stage_elems);
     ULAUNCH();
     return PLATO_OK;
