@@ -1008,31 +1008,62 @@ k_conv_wgrad(TView x, TView dy, float* __restrict__ dW, int cout_real, int32_t p
 
 // ---- element-wise kernels ---------------------------------------------------------------
 
-// masked output gradient (BF16, plain ld = C): m = dy * [y > 0] (relu) or dy
-__global__ void k_grad_mask(TView dy, TView y, int relu, bf16* __restrict__ m, int C, int64_t nvox) {
-    // one thread per (voxel, 4 channels): C, the views' ld and c0 are multiples of 4
-    const int C4 = C / 4;
-    const int64_t total = nvox * C4;
+// Masked output gradient (BF16, plain ld = C, halo zero) m = dy * [y > 0] (relu) or dy, and its sum over
+// the voxels per channel, db[c] += sum m.  One pass over the haloed positions, a thread per (position, 8
+// channels): two 16-byte loads of dy, one of y, one 16-byte store.  The grid stride is a multiple of C / 8, so a
+// thread keeps its channels and sums them in registers; lanes, then warps, then one atomic per channel
+// and block add to db.  Bound by HBM / L2 traffic.  Clearing m, masking and summing in three passes took
+// 13.1 us and 6.8 us a layer on average beside the clear; this pass takes 12.8 us (training step
+// 2.26 -> 2.16 ms).
+__global__ void __launch_bounds__(256) k_grad_mask(TView dy, TView y, int relu, bf16* __restrict__ m, int C, float* __restrict__ db) {
+    __shared__ float sh[8][64];
+    const uint32_t C8 = uint32_t(C) / 8;
+    const uint32_t c = 8 * (threadIdx.x % C8);
+    const uint32_t sy = uint32_t(dy.W + 2), H = uint32_t(dy.H + 2), D = uint32_t(dy.D + 2);
+    const int64_t total = int64_t(dy.B) * D * H * sy * C8;
+    float sum[8] = {};
     for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < total; i += int64_t(gridDim.x) * blockDim.x) {
-        const uint32_t v = uint32_t(i / C4);
-        const int c = 4 * int(i - int64_t(v) * C4);
-        const Vox q = vox_of(dy, v);
-        const int64_t hv = hpos(dy, q.b, q.z, q.y, q.x);
-        const float4 d = *reinterpret_cast<const float4*>(static_cast<const float*>(dy.p) + hv * dy.ld + dy.c0 + c);
-        float val[4] = {d.x, d.y, d.z, d.w};
-        if (relu) {
-            const uint2 yy = *reinterpret_cast<const uint2*>(static_cast<const bf16*>(y.p) + hv * y.ld + y.c0 + c);
-            const __nv_bfloat162 y01 = *reinterpret_cast<const __nv_bfloat162*>(&yy.x);
-            const __nv_bfloat162 y23 = *reinterpret_cast<const __nv_bfloat162*>(&yy.y);
-            if (!(__low2float(y01) > 0.f)) val[0] = 0.f;
-            if (!(__high2float(y01) > 0.f)) val[1] = 0.f;
-            if (!(__low2float(y23) > 0.f)) val[2] = 0.f;
-            if (!(__high2float(y23) > 0.f)) val[3] = 0.f;
+        const uint32_t hv = uint32_t(i / C8);
+        uint32_t t = hv / sy;
+        const uint32_t xx = hv - t * sy;
+        const uint32_t yy = t % H;
+        const uint32_t zz = (t / H) % D;
+        uint4 o = make_uint4(0, 0, 0, 0);
+        if (xx - 1 < uint32_t(dy.W) && yy - 1 < uint32_t(dy.H) && zz - 1 < uint32_t(dy.D)) {
+            const float4* dp = reinterpret_cast<const float4*>(static_cast<const float*>(dy.p) + int64_t(hv) * dy.ld + dy.c0 + c);
+            const float4 a = dp[0], b = dp[1];
+            o = make_uint4(pack_bf16(a.x, a.y), pack_bf16(a.z, a.w), pack_bf16(b.x, b.y), pack_bf16(b.z, b.w));
+            uint32_t* ow = &o.x;
+            if (relu) {
+                const uint4 yv = *reinterpret_cast<const uint4*>(static_cast<const bf16*>(y.p) + int64_t(hv) * y.ld + y.c0 + c);
+                const uint32_t* yw = &yv.x;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162*>(yw + k);
+                    if (!(__low2float(v) > 0.f)) ow[k] &= 0xffff0000u;
+                    if (!(__high2float(v) > 0.f)) ow[k] &= 0x0000ffffu;
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162*>(ow + k);
+                sum[2 * k] += __low2float(v);
+                sum[2 * k + 1] += __high2float(v);
+            }
         }
-        uint2 o;
-        o.x = pack_bf16(val[0], val[1]);
-        o.y = pack_bf16(val[2], val[3]);
-        *reinterpret_cast<uint2*>(m + hv * C + c) = o;
+        *reinterpret_cast<uint4*>(m + int64_t(hv) * C + c) = o;
+    }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        for (uint32_t w = 16; w >= C8; w >>= 1) sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], w);
+        if (uint32_t(lane) < C8) sh[warp][8 * lane + k] = sum[k];
+    }
+    __syncthreads();
+    if (threadIdx.x < uint32_t(C)) {
+        float s = 0.f;
+        for (int w = 0; w < 8; ++w) s += sh[w][threadIdx.x];
+        atomicAdd(db + threadIdx.x, s);
     }
 }
 
@@ -1708,16 +1739,14 @@ int layer_backward(plato_unet* u, int k, TView dy, TView y, TView x, TView dx, b
     const int C = L.coutp() < 16 ? 16 : L.coutp();
     const int gdims[3] = {y.D, y.H, y.W};
     TView m = tv(u->mbuf, C, 0, y.B, gdims);
-    if (k != int(u->layers.size()) - 1) {  // the head's masked gradient is written by the loss
-        // mbuf is reused with other grids and widths: clear it so its halo reads as zero
-        UCUDA(cudaMemsetAsync(u->mbuf, 0, sizeof(bf16) * size_t(halo_elems(gdims, y.B, C)), s));
-        k_grad_mask<<<blocks_for(nvox * L.cout, 256), 256, 0, s>>>(dy, y, L.relu, u->mbuf, C, nvox);
-        ULAUNCH();
-    }
-    URC(conv_weight_grad(s, L, x, m, u->grads + L.w_off, nvox));
     const int64_t mtotal = halo_elems(gdims, y.B, C);
-    k_bias_grad<<<blocks_for(mtotal, 256, 148 * 8), 256, 0, s>>>(u->mbuf, mtotal, C, L.cout, u->grads + L.b_off);
+    if (k != int(u->layers.size()) - 1) {
+        k_grad_mask<<<blocks_for(mtotal / 8, 256, 148 * 8), 256, 0, s>>>(dy, y, L.relu, u->mbuf, C, u->grads + L.b_off);
+    } else {  // the head's masked gradient is written by the loss
+        k_bias_grad<<<blocks_for(mtotal, 256, 148 * 8), 256, 0, s>>>(u->mbuf, mtotal, C, L.cout, u->grads + L.b_off);
+    }
     ULAUNCH();
+    URC(conv_weight_grad(s, L, x, m, u->grads + L.w_off, nvox));
     if (write_dx) URC(conv_data_grad(s, P, L, m, dx, nvox, accumulate));
     return PLATO_OK;
 }
