@@ -841,7 +841,9 @@ constexpr int kWgRows = 128;  // positions per tile (8 k-steps)
 // Warps of a CTA, all on the same staged tile: the kernel waits for ldmatrix and the MMAs most of the
 // time, and shared memory lets three CTAs on an SM, so 8 warps each hide that better than 4, each
 // with one block of 16 output channels (one A fragment per k-step).  Batch 8 on 68x36x36, 48 -> 16 channels
-// 288 -> 163 us, 16 -> 16 79 -> 63 us; 96 -> 32 (34x18x18) 167 -> 92 us.
+// 288 -> 163 us, 16 -> 16 79 -> 63 us; 96 -> 32 (34x18x18) 167 -> 92 us.  With a 16 x 16 tile per ldmatrix.x4,
+// paired atomics and one atomic per CTA instead of one per group of warps 150, 53 and 87 us; the 1x1x1
+// head, whose 144 sums every CTA adds to, 53 (96 with eight groups) -> below 10 us.
 constexpr int kWgWarps = 8, kWgThreads = 32 * kWgWarps;
 
 __device__ __forceinline__ void ldsm_x4_t(uint32_t (&r)[4], const bf16* p) {
@@ -850,19 +852,28 @@ __device__ __forceinline__ void ldsm_x4_t(uint32_t (&r)[4], const bf16* p) {
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                  : "r"(a));
 }
-__device__ __forceinline__ void ldsm_x2_t(uint32_t& r0, uint32_t& r1, const bf16* p) {
-    const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(p));
-    asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];\n" : "=r"(r0), "=r"(r1) : "r"(a));
-}
 
 // tap groups of a weight-gradient launch: the fewest (1, 3, 9 or 27) that leave each warp at most
-// 18 output tiles (72 FP32 sums in registers)
+// 18 output tiles of 16 x 8 (72 FP32 sums in registers)
 template <int CIN, int COUT, int TAPS>
 constexpr int wg_groups() {
     if (TAPS == 1) return 1;
     constexpr int per_tap = (COUT / 16) * (CIN / 8);
     constexpr int most = 18 * kWgWarps;
     return 27 * per_tap <= most ? 1 : 9 * per_tap <= most ? 3 : 3 * per_tap <= most ? 9 : 27;
+}
+
+// Groups of warps that split the k-steps of a launch with T output tiles of 16 x 16 per CTA: all warps on the one
+// tile of the 1x1x1 head, and two groups where four warps share the tiles more evenly than eight (27
+// tiles: 28 places instead of 32; 36: 36 instead of 40) and the sums still fit in registers.
+__host__ __device__ constexpr int wg_ksplit(int T) {
+    return T == 1 ? kWgWarps : 4 * ((T + 3) / 4) < 8 * ((T + 7) / 8) && (T + 3) / 4 <= 9 ? kWgWarps / 4 : 1;
+}
+
+// shared memory that the groups' sums go through at the end
+__host__ __device__ constexpr uint32_t wg_reduce_bytes(int T) {
+    return uint32_t((wg_ksplit(T) - 1) * (kWgWarps / wg_ksplit(T))) * uint32_t((T + kWgWarps / wg_ksplit(T) - 1) / (kWgWarps / wg_ksplit(T))) * 8u * 32u *
+           4u;
 }
 
 // offset of tap t of a 3x3x3 stencil in haloed positions
@@ -884,11 +895,8 @@ k_conv_wgrad(TView x, TView dy, float* __restrict__ dW, int cout_real, int32_t p
     constexpr int TPG = TAPS / G;                         // taps of this CTA
     constexpr int NSL = (TAPS == 27 && G == 1) ? 3 : 1;   // x slabs per tile (one per z offset)
     constexpr int LDY = COUT + 8, LDX = CIN + 8;          // padded rows: 16-byte aligned, no ldmatrix conflicts
-    constexpr int T = TPG * (COUT / 16) * (CIN / 8);      // output tiles of 16 x 8
-    // with at most two output tiles (the 1x1x1 head), groups of warps share a tile and split its
-    // k-steps, so all warps work; each adds its own partial sums
-    constexpr int KSPLIT = T <= 2 ? kWgWarps / 2 : 1;
-    constexpr int WPT = kWgWarps / KSPLIT;
+    constexpr int T = TPG * (COUT / 16) * (CIN / 16);     // output tiles of 16 x 16
+    constexpr int KSPLIT = wg_ksplit(T), WPT = kWgWarps / KSPLIT;
     constexpr int PER = (T + WPT - 1) / WPT;
     extern __shared__ __align__(16) bf16 wg_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -911,16 +919,17 @@ k_conv_wgrad(TView x, TView dy, float* __restrict__ dW, int cout_real, int32_t p
 #pragma unroll
     for (int k = 0; k < PER; ++k) {
         const int id = wt + WPT * k, rest = id / MT;
-        const int j = rest / (CIN / 8), nt = rest - j * (CIN / 8);
+        const int j = rest / (CIN / 16), nt = rest - j * (CIN / 16);
         const int sl = NSL == 3 ? j / 9 : 0;
         const int rel = TAPS == 1 ? 0 : wg_tap_offset(g * TPG + j, sy, sz) - centre[sl];
-        boff[k] = (kWgRows * LDY) + (sl * rows_pad + hw + rel + (lane & 7) + ((lane >> 3) & 1) * 8) * LDX + 8 * nt;
+        boff[k] = (kWgRows * LDY) + (sl * rows_pad + hw + rel + (lane & 7) + ((lane >> 3) & 1) * 8) * LDX + 16 * nt +
+                  8 * (lane >> 4);
     }
-    float acc[PER][4];
+    float acc[PER][2][4];
 #pragma unroll
     for (int k = 0; k < PER; ++k)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) acc[k][q] = 0.f;
+        for (int q = 0; q < 4; ++q) acc[k][0][q] = acc[k][1][q] = 0.f;
     const bf16* __restrict__ yp = static_cast<const bf16*>(dy.p);
     const bf16* __restrict__ xp = static_cast<const bf16*>(x.p);
     const int my_tiles = (ntiles - int(blockIdx.x) + int(gridDim.x) - 1) / int(gridDim.x);
@@ -979,29 +988,40 @@ k_conv_wgrad(TView x, TView dy, float* __restrict__ dW, int cout_real, int32_t p
             for (int q = 0; q < PER; ++q) {
                 if (wt + WPT * q >= T) break;
                 // B = x (rows position, cols ci) at the tap's shifted slab rows
-                uint32_t b0, b1;
-                ldsm_x2_t(b0, b1, sb + boff[q] + 16 * ks * LDX);
-                mma16816(acc[q], a, b0, b1);
+                uint32_t b[4];
+                ldsm_x4_t(b, sb + boff[q] + 16 * ks * LDX);
+                mma16816(acc[q][0], a, b[0], b[1]);
+                mma16816(acc[q][1], a, b[2], b[3]);
             }
         }
         __syncthreads();  // stage k & 1 is refilled by the next iteration's copies
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
+    if constexpr (KSPLIT > 1) {  // the first group adds the others' sums (the stages are free)
+        float* red = reinterpret_cast<float*>(wg_smem) + wt * (PER * 256) + lane;
+        if (kg > 0) {
+#pragma unroll
+            for (int i = 0; i < PER * 8; ++i) red[(kg - 1) * (WPT * PER * 256) + 32 * i] = acc[i >> 3][(i >> 2) & 1][i & 3];
+        }
+        __syncthreads();
+        if (kg > 0) return;
+        for (int o = 0; o < KSPLIT - 1; ++o)
+#pragma unroll
+            for (int i = 0; i < PER * 8; ++i) acc[i >> 3][(i >> 2) & 1][i & 3] += red[o * (WPT * PER * 256) + 32 * i];
+    }
     const int gq = lane >> 2, tig = lane & 3;
 #pragma unroll
     for (int q = 0; q < PER; ++q) {
         const int id = wt + WPT * q;
         if (id >= T) break;
-        const int rest = id / MT, j = rest / (CIN / 8);
-        const int m0 = 16 * mt, n0 = 8 * (rest - j * (CIN / 8));
+        const int rest = id / MT, j = rest / (CIN / 16);
+        const int m0 = 16 * mt, n0 = 16 * (rest - j * (CIN / 16));
         float* w = dW + int64_t(g * TPG + j) * cout_real * CIN;  // rows past the real output channels are padding
-        if (m0 + gq < cout_real) {
-            atomicAdd(w + (m0 + gq) * CIN + n0 + 2 * tig, acc[q][0]);
-            atomicAdd(w + (m0 + gq) * CIN + n0 + 2 * tig + 1, acc[q][1]);
-        }
-        if (m0 + gq + 8 < cout_real) {
-            atomicAdd(w + (m0 + gq + 8) * CIN + n0 + 2 * tig, acc[q][2]);
-            atomicAdd(w + (m0 + gq + 8) * CIN + n0 + 2 * tig + 1, acc[q][3]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {  // two neighbours per atomic: every weight block starts on an even offset
+            const int row = m0 + gq + 8 * (e & 1), col = n0 + 8 * (e >> 1) + 2 * tig;
+            const float* v = &acc[q][e >> 1][2 * (e & 1)];
+            if (row < cout_real) atomicAdd(reinterpret_cast<float2*>(w + row * CIN + col), make_float2(v[0], v[1]));
         }
     }
 }
@@ -1652,7 +1672,8 @@ int wgrad_launch(cudaStream_t s, TView x, TView dy, float* dW, int cout_real, in
     const int srows = kWgRows + 2 * wg_halfwidth<TAPS, G>(int(sy));
     const int rows_pad = srows;
     const uint32_t stage_elems = uint32_t(kWgRows * (COUT + 8) + NSL * rows_pad * (CIN + 8));
-    const uint32_t smem = 2u * stage_elems * 2u;
+    constexpr int T = TAPS / G * (COUT / 16) * (CIN / 16);
+    const uint32_t smem = std::max(2u * stage_elems * 2u, wg_reduce_bytes(T));
     if (smem > 227u * 1024u) return fail(PLATO_NOT_SUPPORTED, "weight gradient: grid rows too long for shared memory");
     auto kernel = k_conv_wgrad<CIN, COUT, TAPS, G>;
     UCUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
