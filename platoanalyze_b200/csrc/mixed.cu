@@ -336,11 +336,27 @@ constexpr int kStHalfBytes = kStK * (576 + 64) + 64;
 constexpr int kStWarpBytes = kStStages * 2 * kStHalfBytes;
 constexpr int kStSmem = (kThreads / 32) * kStWarpBytes;
 
-__device__ __forceinline__ void sweep_cp16(uint32_t dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+// A sweep's matrix that is longer than the L2 (STREAMED) is marked evict-first and so leaves the vectors
+// there, which every step reads again (160x80x80: 320 MB of matrix, 63 MB of vectors): solve and
+// adjoint 38.3 -> 36.3 ms; with an eighth of the slices kept at normal priority 37.1 ms, with a quarter
+// 38.2 ms, so nothing of the matrix is worth keeping; 120x60x60 (136 MB) 19.4 -> 18.3 ms.  One that fits is
+// read without a policy: evict-first costs it 4 % of the solve (100x50x50, 79 MB: 10.9 -> 11.4 ms), and a
+// hint of normal priority, which changes nothing but the instructions, still 2 %.
+__device__ __forceinline__ uint64_t sweep_policy() {
+    uint64_t p;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+template <bool STREAMED>
+__device__ __forceinline__ void sweep_cp16(uint32_t dst, const void* src, uint64_t policy) {
+    if constexpr (STREAMED)
+        asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "l"(policy)
+                     : "memory");
+    else
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 
-template <int MODE>
+template <int MODE, bool STREAMED>
 __global__ void __launch_bounds__(kThreads, 4)
 k_sell16s_st(SellView A, const __half* __restrict__ vals, const float* __restrict__ x, float* __restrict__ res,
              float* __restrict__ dnext, float* __restrict__ y, float c1, float c2, const PcgScalars* S) {
@@ -354,6 +370,7 @@ k_sell16s_st(SellView A, const __half* __restrict__ vals, const float* __restric
                                              reinterpret_cast<uintptr_t>(y)
                                        : uintptr_t(0));
     const bool vec2 = (vbits & 7) == 0;
+    const uint64_t stream = STREAMED ? sweep_policy() : 0;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = lane >> 4, m = lane & 15;
     const uint8_t* wsm = st_smem + warp * kStWarpBytes;
     const uint32_t wsm_s = static_cast<uint32_t>(__cvta_generic_to_shared(wsm));
@@ -380,9 +397,9 @@ k_sell16s_st(SellView A, const __half* __restrict__ vals, const float* __restric
             const int k0 = c * kStK, kn = min(kStK, w - k0);
             if (kn > 0) {
                 const uint32_t dst = wsm_s + uint32_t((stg * 2 + half) * kStHalfBytes);
-                for (int u = m; u < kn * 36; u += 16) sweep_cp16(dst + 16u * u, gv + 576 * int64_t(k0) + 16 * u);
+                for (int u = m; u < kn * 36; u += 16) sweep_cp16<STREAMED>(dst + 16u * u, gv + 576 * int64_t(k0) + 16 * u, stream);
                 for (int u = m; u < kn * 4; u += 16)
-                    sweep_cp16(dst + uint32_t(kStK * 576) + 16u * u, gc + 64 * int64_t(k0) + 16 * u);
+                    sweep_cp16<STREAMED>(dst + uint32_t(kStK * 576) + 16u * u, gc + 64 * int64_t(k0) + 16 * u, stream);
             }
         };
         const int32_t row0 = int32_t(32 * sl);
@@ -1149,6 +1166,7 @@ int fcg_poly(plato_problem* h, const double* b, double* x, plato_solve_stats* st
     // takes 3-4 pairs per thread on the bench mesh): 8 % faster per step than a grid of one
     // pair per thread, whose last partial wave leaves SMs idle.
     int CB = SB, CBst = SB;
+    bool streamed = false;
     if (kind == INNER_SELL16S) {
         int sms = 0, per_sm = 0;
         PLATO_CUDA(h, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
@@ -1156,10 +1174,13 @@ int fcg_poly(plato_problem* h, const double* b, double* x, plato_solve_stats* st
         CB = std::min(SB, std::max(1, per_sm) * std::max(1, sms));
         if (V.dcols) {  // the staged form, one resident wave as well
             int per_st = 0;
-            PLATO_CUDA(h, cudaFuncSetAttribute(k_sell16s_st<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStSmem));
-            PLATO_CUDA(h, cudaFuncSetAttribute(k_sell16s_st<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStSmem));
-            PLATO_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_st, k_sell16s_st<0>, kThreads, kStSmem));
+            for (auto kernel : {k_sell16s_st<0, false>, k_sell16s_st<1, false>, k_sell16s_st<0, true>, k_sell16s_st<1, true>})
+                PLATO_CUDA(h, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStSmem));
+            PLATO_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_st, k_sell16s_st<0, true>, kThreads, kStSmem));
             CBst = std::min(SB, std::max(1, per_st) * std::max(1, sms));
+            int l2 = 0;
+            PLATO_CUDA(h, cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, h->device));
+            streamed = h->sell.total_slots * 20 > l2;  // 9 FP16 entries and a 16-bit offset per slot
         }
     }
     // multi-step sweep (FP16 scaled matrix, numbering with a short column reach)
@@ -1203,7 +1224,7 @@ int fcg_poly(plato_problem* h, const double* b, double* x, plato_solve_stats* st
             k_res_sub_vec<<<VB, kThreads, 0, s>>>(n, h->bc_mask, xin, h->f_w, h->f_res, h->scal);
         } else if (kind == INNER_SELL16S) {
             if (V.dcols)
-                PLATO_CUDA(h, launch_pdl_smem(k_sell16s_st<1>, CBst, kThreads, size_t(kStSmem), s, V,
+                PLATO_CUDA(h, launch_pdl_smem(streamed ? k_sell16s_st<1, true> : k_sell16s_st<1, false>, CBst, kThreads, size_t(kStSmem), s, V,
                                               static_cast<const __half*>(h->sell16s), xin, h->f_res, nullptr, nullptr,
                                               0.f, 0.f, (const PcgScalars*)h->scal));
             else
@@ -1269,7 +1290,7 @@ int fcg_poly(plato_problem* h, const double* b, double* x, plato_solve_stats* st
                                                    cc.c1[k], cc.c2[k], h->scal);
             } else if (kind == INNER_SELL16S) {
                 if (V.dcols)
-                    PLATO_CUDA(h, launch_pdl_smem(k_sell16s_st<0>, CBst, kThreads, size_t(kStSmem), s, V,
+                    PLATO_CUDA(h, launch_pdl_smem(streamed ? k_sell16s_st<0, true> : k_sell16s_st<0, false>, CBst, kThreads, size_t(kStSmem), s, V,
                                                   static_cast<const __half*>(h->sell16s), (const float*)dcur, h->f_res,
                                                   dnext, h->f_y, cc.c1[k], cc.c2[k], (const PcgScalars*)h->scal));
                 else
