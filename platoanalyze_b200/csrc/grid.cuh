@@ -92,6 +92,47 @@ __device__ __forceinline__ bool grid_barrier(const GridBox& a, uint32_t barrier)
     return !__syncthreads_or(!ok);
 }
 
+// The same sum over the CTAs of one cluster (at most 16, the whole grid): each CTA writes its block sums
+// into every CTA's box through distributed shared memory, and the cluster's hardware barrier is the only
+// wait (an iteration with two sums of a 12x6x6 system 7 -> 4.8 us).  The CTAs' threads call it in step; the first
+// call comes after a cluster_barrier(), since a CTA's shared memory exists only once it runs.
+constexpr int kClusterMax = 16;
+
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+template <int NV>
+__device__ __forceinline__ void cluster_sum(double (&v)[NV], uint32_t barrier, double (*sh_cta)[32],
+                                            double (*box)[kGridValues][kClusterMax]) {
+    const int tid = threadIdx.x, w = tid >> 5, l = tid & 31, G = gridDim.x;
+#pragma unroll
+    for (int q = 0; q < NV; ++q) v[q] = warp_sum(v[q]);
+    if (l == 0)
+#pragma unroll
+        for (int q = 0; q < NV; ++q) sh_cta[q][w] = v[q];
+    __syncthreads();
+    if (w == 0) {
+        const int nw = blockDim.x >> 5;
+#pragma unroll
+        for (int q = 0; q < NV; ++q) {
+            const double s = warp_sum(l < nw ? sh_cta[q][l] : 0.0);  // in all lanes
+            if (l < G) {
+                const uint32_t mine = static_cast<uint32_t>(__cvta_generic_to_shared(&box[barrier & 1u][q][blockIdx.x]));
+                uint32_t peer;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(mine), "r"(l));
+                asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(peer), "d"(s) : "memory");
+            }
+        }
+    }
+    cluster_barrier();
+#pragma unroll
+    for (int q = 0; q < NV; ++q) {
+        v[q] = 0.0;
+        for (int i = 0; i < G; ++i) v[q] += box[barrier & 1u][q][i];
+    }
+}
+
 // Cooperative launch of one CTA per SM.
 template <typename Args>
 inline cudaError_t launch_cooperative(void (*kernel)(Args), int grid, int block, size_t smem, cudaStream_t stream,

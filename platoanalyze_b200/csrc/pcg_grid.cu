@@ -11,7 +11,7 @@
 //   x += alpha p, r -= alpha A p, z = Dinv r                 -> sums r.z, r.r          -> beta
 // so two grid-wide sums per iteration, which are also its two barriers.  Only z and p leave the SM.
 // Bound by the two sums (1.5 to 3 us each).  Solve of a cantilever with a random density, launch per stage
-// against this: 20x10x10 15.1 -> 3.2 ms, 30x16x16 24.9 -> 5.2, 40x20x20 30.4 -> 7.5, 60x30x30 54.4 -> 20.6,
+// against this: 20x10x10 15.1 -> 3.2 ms (2.5 as one cluster, see pcg_grid), 30x16x16 24.9 -> 5.2, 40x20x20 30.4 -> 7.5, 60x30x30 54.4 -> 20.6,
 // 64x32x32 84.5 -> 26.4.  Density filter (one unknown per row): 20x10x10 0.66 -> 0.26 ms, 80x40x40
 // 1.92 -> 0.96, 100x50x50 3.30 -> 1.69, 112x53x52 (the largest that qualifies) 4.00 -> 3.81: there the
 // CTAs read the matrix from L2 with two slices per warp, hence the limits in pcg_grid_ok.
@@ -48,10 +48,12 @@ struct GridPcg {
 };
 
 // NB unknowns per row (3: block SELL, 1: scalar SELL), T slices per group of ks warps.
-template <int NB, int T, int THREADS>
+// CLUSTER: the grid is one cluster.
+template <int NB, int T, int THREADS, bool CLUSTER>
 __global__ void __launch_bounds__(THREADS, 1) k_pcg_grid(GridPcg a) {
     extern __shared__ __align__(16) unsigned char grid_smem[];
     __shared__ double sh_cta[2][32], sh_grid[2][32];
+    __shared__ double box[CLUSTER ? 2 : 1][kGridValues][kClusterMax];
     __shared__ double part[NB][THREADS];
     constexpr int NE = NB * NB;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -95,7 +97,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_pcg_grid(GridPcg a) {
     int32_t iter = a.S->iter, done = a.S->done, nonfinite = a.S->nonfinite;
     uint32_t epoch = 0;  // barriers of this launch
     int pcur = a.pcur;
-    __syncthreads();
+    if constexpr (CLUSTER) cluster_barrier();
+    else __syncthreads();
 
     for (int it = 0; it < kLaunchIters && !done; ++it) {
         const double* pold = a.p[pcur];
@@ -143,7 +146,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_pcg_grid(GridPcg a) {
         }
         pcur ^= 1;
         double s1v[1] = {s2[0]};
-        if (!grid_sum<1>(s1v, a.box, ++epoch, sh_cta, sh_grid)) break;
+        if constexpr (CLUSTER) cluster_sum<1>(s1v, ++epoch, sh_cta, box);
+        else if (!grid_sum<1>(s1v, a.box, ++epoch, sh_cta, sh_grid)) break;
         pap = s1v[0];
         alpha = rz / pap;
         if (!isfinite(alpha) || pap <= 0.0) {
@@ -168,7 +172,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_pcg_grid(GridPcg a) {
                 }
             }
         }
-        if (!grid_sum<2>(s2, a.box, ++epoch, sh_cta, sh_grid)) break;
+        if constexpr (CLUSTER) cluster_sum<2>(s2, ++epoch, sh_cta, box);
+        else if (!grid_sum<2>(s2, a.box, ++epoch, sh_cta, sh_grid)) break;
         beta = s2[0] / rz;
         rz = s2[0];
         rr = s2[1];
@@ -206,9 +211,39 @@ constexpr int grid_threads() { return NB == 3 ? 512 : 1024; }
 template <int NB, int T>
 int launch_grid(plato_problem* h, GridPcg& a, int grid) {
     constexpr int THREADS = grid_threads<NB>();
-    const void* kernel = reinterpret_cast<const void*>(k_pcg_grid<NB, T, THREADS>);
-    PLATO_RC(ensure_smem_attribute(h, kernel, a.smem_bytes));
-    PLATO_CUDA(h, launch_cooperative(k_pcg_grid<NB, T, THREADS>, grid, THREADS, size_t(a.smem_bytes), h->stream, a));
+    const auto kernel = k_pcg_grid<NB, T, THREADS, false>;
+    PLATO_RC(ensure_smem_attribute(h, reinterpret_cast<const void*>(kernel), a.smem_bytes));
+    PLATO_CUDA(h, launch_cooperative(kernel, grid, THREADS, size_t(a.smem_bytes), h->stream, a));
+    PLATO_LAUNCH_CHECK(h);
+    return PLATO_OK;
+}
+
+// The launch as one cluster of `grid` CTAs; *ok is cleared, and nothing launched, where the device has no
+// place for it.
+template <int NB>
+int launch_cluster(plato_problem* h, GridPcg& a, int grid, int* ok) {
+    constexpr int THREADS = grid_threads<NB>();
+    const auto kernel = k_pcg_grid<NB, 1, THREADS, true>;
+    PLATO_RC(ensure_smem_attribute(h, reinterpret_cast<const void*>(kernel), a.smem_bytes));
+    PLATO_CUDA(h, cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(unsigned(grid));
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = size_t(a.smem_bytes);
+    cfg.stream = h->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = unsigned(grid);
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess || clusters < 1) {
+        (void)cudaGetLastError();
+        *ok = 0;
+        return PLATO_OK;
+    }
+    PLATO_CUDA(h, cudaLaunchKernelEx(&cfg, kernel, a));
     PLATO_LAUNCH_CHECK(h);
     return PLATO_OK;
 }
@@ -248,8 +283,18 @@ int pcg_grid(plato_problem* h, int nb, const double* vals, const double* dinv, d
     PLATO_CUDA(h, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
     PLATO_CUDA(h, cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h->device));
     const int warps = (nb == 3 ? grid_threads<3>() : grid_threads<1>()) / 32;
-    const int grid = std::min({sms, h->sell.nslices, 32 * warps});
-    const int per_cta = (h->sell.nslices + grid - 1) / grid;
+    const int64_t room = kGridSmemMax - (nb == 3 ? 512 * 24 : 1024 * 8) - 2048;
+    // shared memory for the average CTA's slots and a tenth more; a CTA with more reads L2
+    const auto smem_for = [&](int ctas) { return (h->sell.total_slots / ctas + 32) * (8 * nb * nb + 4) * 11 / 10; };
+    // A system that gives each of 16 SMs its part in shared memory and each slice 3 warps (scalar: one) runs
+    // as one cluster, whose barrier is a hardware one.  One grid-wide counter against this: 12x6x6 2.0 -> 1.4 ms,
+    // 18x9x9 3.0 -> 2.3, 20x10x10 (80 slices, 3 warps each) 3.2 -> 2.5; with 2 warps a slice 21x10x10 3.38 -> 3.41,
+    // so the line lies there.  Filter: 16x8x8 0.49 -> 0.38 ms, 37x20x18 (474 slices, a warp each) 0.97 -> 0.86.
+    int cluster = 1;
+    while (2 * cluster <= std::min<int>(kClusterMax, h->sell.nslices)) cluster *= 2;
+    int clustered = (h->sell.nslices + cluster - 1) / cluster * (nb == 3 ? 3 : 1) <= warps && smem_for(cluster) <= room;
+    int grid = clustered ? cluster : std::min({sms, h->sell.nslices, 32 * warps});
+    int per_cta = (h->sell.nslices + grid - 1) / grid;
     if (!coop || per_cta > 2 * warps || (nb == 3 && per_cta > warps)) {
         PLATO_CUDA(h, cudaMemcpyAsync(h->scal_host, h->scal, sizeof(PcgScalars), cudaMemcpyDeviceToHost, h->stream));
         PLATO_CUDA(h, cudaStreamSynchronize(h->stream));
@@ -260,8 +305,6 @@ int pcg_grid(plato_problem* h, int nb, const double* vals, const double* dinv, d
     GridPcg a{};
     a.A = sell_view(h);
     a.nslices = h->sell.nslices;
-    a.ks = 1;
-    while (2 * a.ks * per_cta <= warps) a.ks *= 2;
     a.vals = vals;
     a.dinv = dinv;
     a.x = x;
@@ -271,12 +314,20 @@ int pcg_grid(plato_problem* h, int nb, const double* vals, const double* dinv, d
     a.p[1] = p2;
     a.max_it = max_it;
     a.S = h->scal;
-    // shared memory for the average CTA's slots and a tenth more; a CTA with more reads L2
-    const int64_t want = (h->sell.total_slots / grid + 32) * (8 * nb * nb + 4) * 11 / 10;
-    a.smem_bytes = want <= kGridSmemMax - (nb == 3 ? 512 * 24 : 1024 * 8) - 2048 ? int((want + 15) / 16 * 16) : 0;
     for (;;) {
+        a.ks = std::max(1, warps / per_cta);
+        const int64_t want = smem_for(grid);
+        a.smem_bytes = want <= room ? int((want + 15) / 16 * 16) : 0;
         PLATO_RC(grid_box(h, &a.box));
-        if (nb == 3) PLATO_RC((launch_grid<3, 1>(h, a, grid)));
+        if (clustered) {
+            if (nb == 3) PLATO_RC(launch_cluster<3>(h, a, grid, &clustered));
+            else PLATO_RC(launch_cluster<1>(h, a, grid, &clustered));
+            if (!clustered) {
+                grid = std::min({sms, h->sell.nslices, 32 * warps});
+                per_cta = (h->sell.nslices + grid - 1) / grid;
+                continue;
+            }
+        } else if (nb == 3) PLATO_RC((launch_grid<3, 1>(h, a, grid)));
         else if (per_cta <= warps) PLATO_RC((launch_grid<1, 1>(h, a, grid)));
         else PLATO_RC((launch_grid<1, 2>(h, a, grid)));
         int32_t abort = 0;

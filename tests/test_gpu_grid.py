@@ -92,6 +92,27 @@ def test_filter_cooperative_matches_launch_per_stage(size):
     assert rel_l2(a.cpu().numpy(), b.cpu().numpy()) <= 1e-10 and rel_l2(g.cpu().numpy(), h.cpu().numpy()) <= 1e-10
 
 
+@pytest.mark.parametrize("size", [(4, 3, 3), (9, 5, 5), (13, 6, 6), (18, 9, 9), (21, 10, 10)], ids=lambda s: "x".join(map(str, s)))
+def test_cluster_matches_launch_per_stage(size):
+    """Systems that run as one thread-block cluster: 2, 8 and 16 CTAs, ragged shares, and the first size beyond;
+    the scalar filter on the same meshes (and its own bars)."""
+    spec = cantilever(*size, method_options("plain", 1e-10, (2, 1, 1)))
+    z = splitmix_uniform(spec.coords.shape[0], 3, 0.2, 1.0)
+    p = EllipticProblem(spec)
+    f = HelmholtzFilter(spec.coords, spec.connectivity, 0.08)
+    got = []
+    for timing in (False, True):
+        p.set_timing(timing)
+        f.set_timing(timing)
+        u, st = p.solution(p.to_dev(z))
+        assert st["converged"] and st["fallback"] == 0 and st["relative_residual"] <= 1e-10, st
+        got.append((st["iterations"], u.cpu().numpy(), f.solution(f.to_dev(z))[0].cpu().numpy()))
+    (a, u, c), (b, v, d) = got
+    assert abs(a - b) <= max(3, b // 20) and rel_l2(u, v) <= 1e-8 and rel_l2(c, d) <= 1e-10
+    uo, _, _ = Oracle.from_spec(spec).solution_refined(z, tol=1e-13)
+    assert rel_l2(u, uo) <= 1e-8
+
+
 def test_multistep_sweep_beyond_the_cooperative_range():
     """The multi-step sweep kernel serves the systems that the cooperative loop leaves to it: the same
     arithmetic per row as one launch per step, so the same iterations and solution."""
