@@ -23,7 +23,12 @@
 // accumulator is [slot][component][lane ^ component]: in the accumulation every lane
 // touches the same component at a time, so the 64-bit accesses of a half warp hit 16
 // distinct bank pairs; in the row-major write-out (CRS) 16 consecutive entries of one row
-// span at most 9 components, two to a bank pair.
+// span at most 9 components, two to a bank pair.  The CRS output's transposes and diagonal blocks go out
+// nine lanes to a block as well: a store of one value of 32 blocks touches 32 lines, three whole
+// blocks 3 to 6.  Coordinates are read from planes (a warp's 32 consecutive rows see 2 to 3 lines a load
+// instead of 6).  CRS of 120x60x60: 471 -> 441 us; bound by latency with the 12 warps that the registers
+// allow.  Incidence entries laid out slice-major were slower (491 us): a lane's own entries share
+// a line that stays in L1, a slice's next entries come from L2.
 //
 // Rows with more than kAsmMaxUp upper blocks or more than 255 blocks (high-valence nodes of
 // general meshes) are "wide": skipped here and assembled whole, with the transposes of their
@@ -153,7 +158,7 @@ __device__ __forceinline__ void store_sell(const SellOut& so, int64_t o, double 
 // 9 x 32 x up values and the CTA as many warps as the shared memory takes (at most 14).
 template <bool kSell, typename T>
 __global__ void __launch_bounds__(kAsmMaxWarps * 32, 1)
-k_assemble_rows(MeshView m, GraphView g, Material mat, const double* __restrict__ z,
+k_assemble_rows(MeshView m, const double* __restrict__ px, GraphView g, Material mat, const double* __restrict__ z,
                 const uint16_t* __restrict__ plan, const uint8_t* __restrict__ mirror,
                 const uint8_t* __restrict__ wide, int up, double* __restrict__ crs, SellOut so) {
     const int nwarps = blockDim.x >> 5;
@@ -161,6 +166,7 @@ k_assemble_rows(MeshView m, GraphView g, Material mat, const double* __restrict_
     T* smem = reinterpret_cast<T*>(smem_raw);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     T* acc = smem + warp * (9 * 32 * up);
+    const double *py = px + g.num_nodes, *pz = py + g.num_nodes;  // coordinate planes
     const T lam = T(mat.c01), mu = T(mat.c33);
     const int32_t nslices = (g.num_nodes + 31) >> 5;
     for (int32_t s = blockIdx.x * nwarps + warp; s < nslices; s += gridDim.x * nwarps) {
@@ -175,9 +181,9 @@ k_assemble_rows(MeshView m, GraphView g, Material mat, const double* __restrict_
                 kc = g.n2c_ptr[r + 1] - ks;
                 dslot = g.diag[r] - rs;
                 nup = nb - dslot - 1;
-                xr[0] = T(__ldg(m.coords + 3 * (int64_t)r));
-                xr[1] = T(__ldg(m.coords + 3 * (int64_t)r + 1));
-                xr[2] = T(__ldg(m.coords + 3 * (int64_t)r + 2));
+                xr[0] = T(__ldg(px + r));
+                xr[1] = T(__ldg(py + r));
+                xr[2] = T(__ldg(pz + r));
                 zr = mat.cell_control ? T(0) : T(__ldg(z + r));
             }
         }
@@ -200,12 +206,9 @@ k_assemble_rows(MeshView m, GraphView g, Material mat, const double* __restrict_
             const int32_t i0 = la == 0 ? nk.y : nk.x;
             const int32_t i1 = la <= 1 ? nk.z : nk.y;
             const int32_t i2 = la <= 2 ? nk.w : nk.z;
-            const double* c0 = m.coords + 3 * (int64_t)i0;
-            const double* c1 = m.coords + 3 * (int64_t)i1;
-            const double* c2 = m.coords + 3 * (int64_t)i2;
-            cx[0] = __ldg(c0); cx[1] = __ldg(c0 + 1); cx[2] = __ldg(c0 + 2);
-            cx[3] = __ldg(c1); cx[4] = __ldg(c1 + 1); cx[5] = __ldg(c1 + 2);
-            cx[6] = __ldg(c2); cx[7] = __ldg(c2 + 1); cx[8] = __ldg(c2 + 2);
+            cx[0] = __ldg(px + i0); cx[1] = __ldg(py + i0); cx[2] = __ldg(pz + i0);
+            cx[3] = __ldg(px + i1); cx[4] = __ldg(py + i1); cx[5] = __ldg(pz + i1);
+            cx[6] = __ldg(px + i2); cx[7] = __ldg(py + i2); cx[8] = __ldg(pz + i2);
             if (mat.cell_control) {
                 cz[0] = __ldg(z + (pk >> 2));
                 cz[1] = cz[2] = 0.0;
@@ -376,23 +379,24 @@ k_assemble_rows(MeshView m, GraphView g, Material mat, const double* __restrict_
                         K[3 * i + jj] = lam * S[3 * i + jj] + mu * S[3 * jj + i] + (i == jj ? tr : T(0));
 #pragma unroll
                 for (int q = 0; q < 9; ++q) acc[acc_index<kSell>(u, q, lane)] = K[q];
-                const int k = dslot + 1 + u;
-                const uint8_t ms = __ldg(mirror + rs + k);
-                if (ms != kNoMirror) {
-                    const int32_t c = __ldg(g.cols + rs + k);
-                    double* dst = crs + 9 * ((int64_t)__ldg(g.row_map + c) + ms);
-#pragma unroll
-                    for (int i = 0; i < 3; ++i)
-#pragma unroll
-                        for (int jj = 0; jj < 3; ++jj) dst[3 * i + jj] = double(K[3 * jj + i]);
-                }
-            }
-            if (dslot >= 0) {
-                double* dst = crs + 9 * ((int64_t)rs + dslot);
-#pragma unroll
-                for (int q = 0; q < 9; ++q) dst[q] = double(Kd[q]);
             }
             __syncwarp();
+            // the transposes into rows c: nine lanes write a block, three blocks per store
+            const int wg = lane / 9, wq = lane - 9 * wg, wt = 3 * (wq % 3) + wq / 3;
+            for (int u = 0; u < nupw; ++u) {
+                int32_t blk = -1;  // this row's block in row c
+                if (u < nup) {
+                    const int k = dslot + 1 + u;
+                    const uint8_t ms = __ldg(mirror + rs + k);
+                    if (ms != kNoMirror) blk = __ldg(g.row_map + __ldg(g.cols + rs + k)) + ms;
+                }
+#pragma unroll
+                for (int l0 = 0; l0 < 32; l0 += 3) {
+                    const int l = l0 + wg;
+                    const int32_t b = __shfl_sync(0xffffffffu, blk, l & 31);
+                    if (wg < 3 && l < 32 && b >= 0) crs[9 * (int64_t)b + wq] = double(acc[acc_index<kSell>(u, wt, l)]);
+                }
+            }
             // row-major write-out of the upper blocks: one contiguous run per row
             for (int l = 0; l < 32; ++l) {
                 const int nv = 9 * __shfl_sync(0xffffffffu, nup, l);
@@ -403,6 +407,18 @@ k_assemble_rows(MeshView m, GraphView g, Material mat, const double* __restrict_
                     const int q = e % 9;
                     dst[e] = double(acc[e * 32 + (l ^ q)]);
                 }
+            }
+            __syncwarp();
+            // the diagonal blocks in the same way, through slot 0
+#pragma unroll
+            for (int q = 0; q < 9; ++q) acc[acc_index<kSell>(0, q, lane)] = Kd[q];
+            __syncwarp();
+            const int32_t blk = dslot >= 0 ? rs + dslot : -1;
+#pragma unroll
+            for (int l0 = 0; l0 < 32; l0 += 3) {
+                const int l = l0 + wg;
+                const int32_t b = __shfl_sync(0xffffffffu, blk, l & 31);
+                if (wg < 3 && l < 32 && b >= 0) crs[9 * (int64_t)b + wq] = double(acc[acc_index<kSell>(0, wq, l)]);
             }
         }
         __syncwarp();
@@ -460,7 +476,7 @@ int launch_assemble_jacobian(plato_problem* h, const double* z, double* entries)
     int grid = 0, threads = 0, smem = 0;
     PLATO_RC(asm_launch(h, reinterpret_cast<const void*>(k_assemble_rows<false, double>), sizeof(double), &grid,
                         &threads, &smem));
-    k_assemble_rows<false, double><<<grid, threads, smem, h->stream>>>(mesh_view(h), graph_view(h), h->material, z,
+    k_assemble_rows<false, double><<<grid, threads, smem, h->stream>>>(mesh_view(h), h->coords_soa, graph_view(h), h->material, z,
                                                                       h->asm_plan, h->asm_mirror, h->asm_wideflag,
                                                                       h->asm_maxup, entries, SellOut{});
     PLATO_LAUNCH_CHECK(h);
@@ -489,7 +505,7 @@ int launch_assemble_sell(plato_problem* h, const double* z, double* v64, float* 
     SellOut so{h->sell.ptr, h->sell.cols, h->bc_mask, v64, v32, static_cast<__nv_bfloat16*>(v16), dinv, dinv32};
     // the solver's assembly timing (instrumentation) brackets this one kernel
     if (h->timing && h->asm_ev[0]) PLATO_CUDA(h, cudaEventRecord(h->asm_ev[0], h->stream));
-    k_assemble_rows<true, double><<<grid, threads, smem, h->stream>>>(mesh_view(h), graph_view(h), h->material, z,
+    k_assemble_rows<true, double><<<grid, threads, smem, h->stream>>>(mesh_view(h), h->coords_soa, graph_view(h), h->material, z,
                                                                      h->asm_plan, h->asm_mirror, h->asm_wideflag,
                                                                      h->asm_maxup, nullptr, so);
     PLATO_LAUNCH_CHECK(h);
@@ -507,7 +523,7 @@ int launch_assemble_sell32(plato_problem* h, const double* z, float* v32, float*
     PLATO_RC(asm_launch(h, reinterpret_cast<const void*>(k_assemble_rows<true, float>), sizeof(float), &grid,
                         &threads, &smem));
     SellOut so{h->sell.ptr, h->sell.cols, h->bc_mask, nullptr, v32, nullptr, nullptr, dinv32};
-    k_assemble_rows<true, float><<<grid, threads, smem, h->stream>>>(mesh_view(h), graph_view(h), h->material, z,
+    k_assemble_rows<true, float><<<grid, threads, smem, h->stream>>>(mesh_view(h), h->coords_soa, graph_view(h), h->material, z,
                                                                     h->asm_plan, h->asm_mirror, h->asm_wideflag,
                                                                     h->asm_maxup, nullptr, so);
     PLATO_LAUNCH_CHECK(h);
