@@ -420,10 +420,15 @@ k_conv_tc(TView in, const bf16* __restrict__ Wt, const float* __restrict__ bias,
                         }
                         *reinterpret_cast<float4*>(op + j) = w4;
                     }
-                } else {
+                } else {  // the head's 9 channels of 16: whole vectors, zero past the last channel (9 scalar
+                          // stores a row: 46 -> 26 us at batch 8 on 68x36x36)
+                    static_assert(COUT % 16 == 0 || !OUT_F32 || !ACCUM, "a ragged channel count is written, not added to");
 #pragma unroll
-                    for (int j = 0; j < 16; ++j)
-                        if (c0 + j < COUT) op[j] = ACCUM ? op[j] + y[j] : y[j];
+                    for (int j = 0; j < 16; j += 4)
+                        if (c0 + j < COUT)
+                            *reinterpret_cast<float4*>(op + j) =
+                                make_float4(y[j], c0 + j + 1 < COUT ? y[j + 1] : 0.f, c0 + j + 2 < COUT ? y[j + 2] : 0.f,
+                                            c0 + j + 3 < COUT ? y[j + 3] : 0.f);
                 }
             } else {
                 bf16* op = static_cast<bf16*>(out.p) + obase + c0;
@@ -843,7 +848,7 @@ constexpr int kWgRows = 128;  // positions per tile (8 k-steps)
 // with one block of 16 output channels (one A fragment per k-step).  Batch 8 on 68x36x36, 48 -> 16 channels
 // 288 -> 163 us, 16 -> 16 79 -> 63 us; 96 -> 32 (34x18x18) 167 -> 92 us.  With a 16 x 16 tile per ldmatrix.x4,
 // paired atomics and one atomic per CTA instead of one per group of warps 150, 53 and 87 us; the 1x1x1
-// head, whose 144 sums every CTA adds to, 53 (96 with eight groups) -> below 10 us.
+// head, whose 144 sums every CTA adds to, 53 (96 with eight groups) -> 17 us.
 constexpr int kWgWarps = 8, kWgThreads = 32 * kWgWarps;
 
 __device__ __forceinline__ void ldsm_x4_t(uint32_t (&r)[4], const bf16* p) {
@@ -1252,7 +1257,7 @@ __global__ void k_unpack_output(TView out, int n0, int n1, int n2, float* __rest
 // mean squared error over the node region and its gradient (zero on padding voxels); one
 // thread per voxel of the padded grid: the 16-channel output row in four float4 loads, the
 // BF16 gradient row in two 16-byte stores
-__global__ void k_loss(TView out, const float* __restrict__ tgt, int n0, int n1, int n2, TView dout,
+__global__ void __launch_bounds__(256) k_loss(TView out, const float* __restrict__ tgt, int n0, int n1, int n2, TView dout,
                        double* __restrict__ loss) {
     const int64_t nv = int64_t(out.B) * out.D * out.H * out.W;
     const double inv = 1.0 / (double(out.B) * n0 * n1 * n2 * 9);
@@ -1289,8 +1294,15 @@ __global__ void k_loss(TView out, const float* __restrict__ tgt, int n0, int n1,
         drow[0] = lo;
         drow[1] = hi;
     }
+    // one atomic per block: with one per warp of 4,736 blocks the single address took 20 us
+    __shared__ double sh[8];
     for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss, local * inv);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = local;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) local += sh[w];
+        atomicAdd(loss, local * inv);
+    }
 }
 
 // Adam (Kingma & Ba) on the FP32 parameters
@@ -1306,18 +1318,31 @@ __global__ void k_adam(int64_t n, float* __restrict__ p, const float* __restrict
     }
 }
 
-// BF16 copies of a layer's weights: forward [t][co][ci] and data-gradient [t'][ci][co]
-// with t' = taps - 1 - t (flipped kernel, transposed channels)
-__global__ void k_pack_weights(const float* __restrict__ w, int taps, int cout, int coutp, int cin,
-                               bf16* __restrict__ wf, bf16* __restrict__ wb, int cinp_b) {
-    const int64_t n = int64_t(taps) * coutp * cin;
-    for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
-        const int ci = int(i % cin);
-        const int co = int((i / cin) % coutp);
-        const int t = int(i / (int64_t(cin) * coutp));
-        const float val = co < cout ? w[(int64_t(t) * cout + co) * cin + ci] : 0.f;
-        wf[i] = __float2bfloat16(val);
-        if (wb && co < cinp_b) wb[(int64_t(taps - 1 - t) * cin + ci) * cinp_b + co] = __float2bfloat16(val);
+// BF16 copies of the layers' weights: forward [t][co][ci] and data-gradient [t'][ci][co]
+// with t' = taps - 1 - t (flipped kernel, transposed channels).  One launch for all layers (a launch each:
+// 28 us of a training step, and as many gaps).
+struct PackLayer {
+    const float* w;
+    bf16 *wf, *wb;
+    int taps, cout, coutp, cin, cinp_b;
+    int first;  // running number of its first weight
+};
+constexpr int kMaxLayers = 16;
+struct PackAll {
+    PackLayer layer[kMaxLayers];
+    int n, total;
+};
+
+__global__ void k_pack_weights(const __grid_constant__ PackAll a) {
+    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < a.total; g += gridDim.x * blockDim.x) {
+        int q = 0;
+        while (q + 1 < a.n && g >= a.layer[q + 1].first) ++q;
+        const PackLayer& L = a.layer[q];
+        const int i = g - L.first;
+        const int ci = i % L.cin, co = (i / L.cin) % L.coutp, t = i / (L.cin * L.coutp);
+        const float val = co < L.cout ? L.w[(int64_t(t) * L.cout + co) * L.cin + ci] : 0.f;
+        L.wf[i] = __float2bfloat16(val);
+        if (L.wb && co < L.cinp_b) L.wb[(int64_t(L.taps - 1 - t) * L.cin + ci) * L.cinp_b + co] = __float2bfloat16(val);
     }
 }
 
@@ -1705,13 +1730,14 @@ int conv_weight_grad(cudaStream_t s, const Layer& L, TView x, TView dy, float* d
     } while (0)
 
 int pack_all_weights(plato_unet* u) {
+    PackAll a{};
+    if (u->layers.size() > size_t(kMaxLayers)) return fail(PLATO_NOT_SUPPORTED, "more layers than the weight packing holds");
     for (Layer& L : u->layers) {
-        const int64_t n = int64_t(L.taps) * L.coutp() * L.cin;
-        const int cinp_b = L.taps == 1 ? 16 : L.coutp();
-        k_pack_weights<<<blocks_for(n, 256), 256, 0, u->stream>>>(u->params + L.w_off, L.taps, L.cout, L.coutp(), L.cin,
-                                                                 L.wf, L.wb, cinp_b);
-        ULAUNCH();
+        a.layer[a.n++] = {u->params + L.w_off, L.wf, L.wb, L.taps, L.cout, L.coutp(), L.cin, L.taps == 1 ? 16 : L.coutp(), a.total};
+        a.total += L.taps * L.coutp() * L.cin;
     }
+    k_pack_weights<<<blocks_for(a.total, 256), 256, 0, u->stream>>>(a);
+    ULAUNCH();
     return PLATO_OK;
 }
 
@@ -1986,7 +2012,7 @@ int plato_unet_loss_and_gradients(plato_unet* u, int32_t batch, const float* inp
     UCUDA(cudaMemsetAsync(u->loss_d, 0, sizeof(double), s));
     UCUDA(cudaMemsetAsync(u->mbuf, 0, sizeof(bf16) * size_t(halo_elems(u->g0, batch, 16)), s));
     const int64_t n0 = int64_t(batch) * u->g0[0] * u->g0[1] * u->g0[2];
-    k_loss<<<blocks_for(n0, 256), 256, 0, s>>>(tv(u->out, 16, 0, batch, u->g0), target, u->n[0], u->n[1], u->n[2],
+    k_loss<<<blocks_for(n0, 256, 148 * 8), 256, 0, s>>>(tv(u->out, 16, 0, batch, u->g0), target, u->n[0], u->n[1], u->n[2],
                                                    tv(u->mbuf, 16, 0, batch, u->g0), u->loss_d);
     ULAUNCH();
     URC(backward(u, batch));
