@@ -57,10 +57,10 @@ TRAFFIC_RATIO = {
     "sweep": (150.34 + 3.67) / 166.35,  # k_sell16s_st<0> (16-bit columns)
     "fp64_spmv": 533.8 / 525.52,    # k_fcg_sell_apply
     "assembly": 595.5 / 559.79,     # k_assemble_rows<SELL>
-    "residual": 79.58 / 77.49,      # k_internal_force
-    "energy": 67.58 / 66.69,        # k_energy_sum
-    "dcdz": 135.35 / 70.29,         # k_cell_quantity<2> + k_node_sum
-    "criterion": 135.34 / 70.29,    # k_energy_and_cell_grad + k_node_sum
+    "residual": 99.0 / 77.49,       # k_fans<FAN_FORCE> + k_fan_nodes<3>
+    "energy": 39.1 / 66.69,         # k_fans<FAN_QUANT, 0>
+    "dcdz": 67.7 / 70.29,           # k_fans<FAN_QUANT, 2> + k_fan_nodes<1>
+    "criterion": 67.9 / 70.29,      # k_fans<FAN_QUANT, 5> + k_fan_nodes<1>
 }
 TRAFFIC_NOTE = "ncu DRAM bytes per launch on the 120x60x60 cantilever, scaled by the algorithmic bytes"
 
@@ -772,13 +772,13 @@ def main():
                 "avg_launch_ms": ms, "launches_timed": count}
 
     rl_elements = {
-        "residual": roof_line("k_internal_force (+ the load copy): R = K(z) u - F", elem_in + 24 * N,
+        "residual": roof_line("k_fans<FAN_FORCE> + k_fan_nodes<3>: R = K(z) u - F", elem_in + 24 * N,
                               inst_e["residual_ms_total"], inst_e["residual_timed"], TRAFFIC_RATIO["residual"]),
-        "energy": roof_line("k_energy_sum: compliance 1/2 u^T K(z) u", elem_in,
+        "energy": roof_line("k_fans<FAN_QUANT, 0>: compliance 1/2 u^T K(z) u", elem_in,
                             inst_e["energy_ms_total"], inst_e["energy_timed"], TRAFFIC_RATIO["energy"]),
-        "dcdz": roof_line("k_cell_quantity<2> + k_node_sum: self-adjoint dC/dz", elem_in + 8 * N,
+        "dcdz": roof_line("k_fans<FAN_QUANT, 2> + k_fan_nodes<1>: self-adjoint dC/dz", elem_in + 8 * N,
                           inst_e["dcdz_ms_total"], inst_e["dcdz_timed"], TRAFFIC_RATIO["dcdz"]),
-        "criterion_in_step": roof_line("k_energy_and_cell_grad + k_node_sum: compliance and dC/dz in one pass "
+        "criterion_in_step": roof_line("k_fans<FAN_QUANT, 5> + k_fan_nodes<1>: compliance and dC/dz in one pass "
                                        "(the step's ComputeCriterion)", elem_in + 8 * N,
                                        inst["criterion_ms_total"], inst["criterion_timed"],
                                        TRAFFIC_RATIO["criterion"])}
