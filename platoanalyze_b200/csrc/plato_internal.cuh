@@ -141,6 +141,7 @@ constexpr int kFanMaxCtas = 148 * 32;  // CTAs of an element kernel
 struct FanPlan {
     int       ready = 0;
     int32_t   nfans = 0, ntiles = 0, width = 0;
+    void*     mem[2] = {nullptr, nullptr};  // the arrays below, in two allocations (weights apart)
     int32_t*  rec = nullptr;
     int32_t*  cells = nullptr;
     int32_t*  tile_ptr = nullptr;
