@@ -102,3 +102,15 @@ def test_element_kernels(name):
     close(p.vf_value(ud, zed), orc.vf_value(u, ze))
     close(p.sf_gradient_z(ud, zed), orc.sf_gradient_z(u, ze))
     close(np.array([p.sf_value(ud, zed), p.volume_value(zed)]), np.array([orc.sf_value(u, ze), orc.volume_value(ze)]))
+
+
+@pytest.mark.parametrize("name", MESHES)
+def test_jacobian_write_out(name):
+    """The block CRS Jacobian's shared write-out (nine lanes to a block) on the same meshes: ragged last slices,
+    rows without upper blocks, rows beyond the row kernel's range.  Sums over a node's cells: the same bar."""
+    x, conn = MESHES[name]()
+    spec = ProblemSpec(x, conn, 1.7, 0.28, 3.0, 1e-9, [], np.array([0, 1, 5], np.int32), np.zeros(3))
+    p, orc = EllipticProblem(spec), Oracle.from_spec(spec)
+    z = splitmix_uniform(x.shape[0], 5, 0.3, 1.0)
+    u = np.zeros(3 * x.shape[0])
+    close(p.vf_gradient_u(p.to_dev(u), p.to_dev(z)).reshape(-1), np.asarray(orc.vf_gradient_u(u, z)).reshape(-1))

@@ -128,3 +128,17 @@ def test_multistep_sweep_beyond_the_cooperative_range():
         got.append((st["iterations"], u.cpu().numpy()))
     for it, u in got[1:]:
         assert it == got[0][0] and rel_l2(u, got[0][1]) <= 1e-14  # the bar of the small meshes' test
+
+
+@pytest.mark.parametrize("size", [(112, 56, 56), (120, 60, 60)], ids=lambda s: "x".join(map(str, s)))
+def test_sweep_on_both_sides_of_the_l2(size):
+    """The FP16 sweep with a matrix that fits in the L2 and with one that is read evict-first: both solves meet
+    the tolerance that the FP32 sweep's solve of the same system meets."""
+    got = []
+    for method in ("two-level-fp16", "two-level"):
+        spec = cantilever(*size, method_options(method, 1e-10, coarse_grid(*size)))
+        p = EllipticProblem(spec)
+        u, st = p.solution(p.to_dev(splitmix_uniform(p.num_nodes, 3, 0.2, 1.0)))
+        assert st["converged"] and st["fallback"] == 0 and st["relative_residual"] <= 1e-10, st
+        got.append(u.cpu().numpy())
+    assert rel_l2(*got) <= 1e-8
