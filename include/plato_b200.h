@@ -214,6 +214,13 @@ int plato_get_sweep_info(const plato_problem* h, int32_t* steps_per_launch, int3
  * the solve reports the timeout to the host, the multi-step sweep is switched off for the
  * handle and the plain FP64 Jacobi-PCG fallback finishes the solve (fallback_max_iterations). */
 int plato_test_stall_next_sweep(plato_problem* h);
+/* Test hook (no reference counterpart): how the cooperative Jacobi-PCG lays a system of nslices slices of
+ * 32 rows, total_slots slots in all, over `sms` SMs (without a device): out = {CTAs, slices of the largest
+ * share, warps per slice, slices a group of warps takes in turn, 1 if the matrix is kept in shared
+ * memory, highest index read of a CTA's partial sums (16 warps of 32 entries with 3 unknowns per row, 32
+ * warps with 1; -1: none read)}. */
+int plato_test_pcg_split(int32_t nslices, int64_t total_slots, int32_t unknowns_per_row, int32_t sms, int32_t may_cluster,
+                         int32_t out[6]);
 /* The solver's SELL-32 layout of the block matrix: slots (blocks plus the padding of each
  * 32-row slice to its widest row) and the bytes per column index the FP16 preconditioner
  * sweep reads (2 when every column lies within 32767 of its slice's first row, else 4). */

@@ -41,6 +41,7 @@ int launch_masked_axpy(plato_problem* h, double a, const double* x, double* y);
 int launch_constrained_apply(plato_problem* h, const double* z, const double* x, double* y);
 int launch_sell_spmv(plato_problem* h, const double* vals, const double* x, double* y);
 int launch_coords_soa(plato_problem* h);
+void pcg_split_info(int nslices, int64_t total_slots, int nb, int sms, bool may_cluster, int32_t out[6]);
 int launch_volume(plato_problem* h, const Material& pen, const double* z, double* result);
 int launch_volume_gradient(plato_problem* h, const Material& pen, const double* z, double* dvdz);
 }  // namespace plato
@@ -453,6 +454,14 @@ int plato_get_kernel_timing(const plato_problem* hc, int32_t kind, double* ms_to
 int plato_test_stall_next_sweep(plato_problem* h) {
     if (!h) return PLATO_BAD_INPUT;
     h->wave_stall = 1;
+    return PLATO_OK;
+}
+
+int plato_test_pcg_split(int32_t nslices, int64_t total_slots, int32_t unknowns_per_row, int32_t sms, int32_t may_cluster,
+                         int32_t out[6]) {
+    if (!out || nslices < 1 || total_slots < 32 || sms < 1 || (unknowns_per_row != 1 && unknowns_per_row != 3))
+        return PLATO_BAD_INPUT;
+    pcg_split_info(nslices, total_slots, unknowns_per_row, sms, may_cluster != 0, out);
     return PLATO_OK;
 }
 

@@ -150,6 +150,18 @@ inline cudaError_t launch_cooperative(void (*kernel)(Args), int grid, int block,
     return cudaLaunchKernelEx(&cfg, kernel, args);
 }
 
+// What a warp does in a CTA whose `warps` warps form groups of `parts`, a group per slice: its part of the
+// slice and its group.  Where `parts` does not divide `warps`, the warps that are left over belong to no
+// group and lead none.
+struct WarpRole {
+    int  part, group;
+    bool leader;  // keeps the rows' vectors and adds the other parts' sums to its own
+};
+__host__ __device__ __forceinline__ WarpRole warp_role(int warp, int parts, int warps) {
+    const int group = warp / parts, part = warp - group * parts;
+    return {part, group, part == 0 && group < warps / parts};
+}
+
 // The boxes, counter (cleared for the next launch) and abort flag of a handle (pcg_grid.cu).
 int grid_box(plato_problem* h, GridBox* box);
 

@@ -58,8 +58,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_pcg_grid(GridPcg a) {
     constexpr int NE = NB * NB;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int s0 = int((int64_t)a.nslices * blockIdx.x / gridDim.x), s1 = int((int64_t)a.nslices * (blockIdx.x + 1) / gridDim.x);
-    const int kg = warp % a.ks, group = warp / a.ks, groups = (THREADS / 32) / a.ks;
-    const bool leader = kg == 0;
+    const WarpRole role = warp_role(warp, a.ks, THREADS / 32);
+    const int kg = role.part, group = role.group, groups = (THREADS / 32) / a.ks;
+    const bool leader = role.leader;
 
     // this CTA's slots in shared memory, when they fit
     const int64_t first = a.A.ptr[s0], slots = a.A.ptr[s1] - first;
@@ -274,6 +275,58 @@ bool pcg_grid_ok(const plato_problem* h, int nb) {
     return h->sell.nslices <= int64_t(kNumSMs) * warps * (nb == 3 ? 1 : 2);
 }
 
+namespace {
+
+// How a system of nslices slices with total_slots slots is laid over the SMs.
+struct PcgSplit {
+    int     grid, clustered;
+    int     per_cta;     // slices of the largest share
+    int     ks;          // warps per slice
+    int     turns;       // slices a group of warps takes one after the other
+    int64_t smem_bytes;  // dynamic shared memory (0: the matrix is read from L2)
+};
+
+PcgSplit pcg_split(int nslices, int64_t total_slots, int nb, int sms, bool may_cluster) {
+    const int warps = (nb == 3 ? grid_threads<3>() : grid_threads<1>()) / 32;
+    const int64_t room = kGridSmemMax - (nb == 3 ? 512 * 24 : 1024 * 8) - 2048;
+    // shared memory for the average CTA's slots and a tenth more; a CTA with more reads L2
+    const auto smem_for = [&](int ctas) { return (total_slots / ctas + 32) * (8 * nb * nb + 4) * 11 / 10; };
+    // A system that gives each of 16 SMs its part in shared memory and each slice 3 warps (scalar: one) runs
+    // as one cluster, whose barrier is a hardware one.  One grid-wide counter against this: 12x6x6 2.0 -> 1.4 ms,
+    // 18x9x9 3.0 -> 2.3, 20x10x10 (80 slices, 3 warps each) 3.2 -> 2.5; with 2 warps a slice 21x10x10 3.38 -> 3.41,
+    // so the line lies there.  Filter: 16x8x8 0.49 -> 0.38 ms, 37x20x18 (474 slices, a warp each) 0.97 -> 0.86.
+    int cluster = 1;
+    while (2 * cluster <= std::min<int>(kClusterMax, nslices)) cluster *= 2;
+    PcgSplit p{};
+    p.clustered = may_cluster && (nslices + cluster - 1) / cluster * (nb == 3 ? 3 : 1) <= warps && smem_for(cluster) <= room;
+    p.grid = p.clustered ? cluster : std::min({sms, nslices, 32 * warps});
+    p.per_cta = (nslices + p.grid - 1) / p.grid;
+    p.ks = std::max(1, warps / p.per_cta);
+    p.turns = (p.per_cta + warps / p.ks - 1) / (warps / p.ks);
+    const int64_t want = smem_for(p.grid);
+    p.smem_bytes = want <= room ? (want + 15) / 16 * 16 : 0;
+    return p;
+}
+
+}  // namespace
+
+// The split of a system and the highest index that its kernel's leaders read of the array of partial sums
+// (a CTA has as many entries as threads).
+void pcg_split_info(int nslices, int64_t total_slots, int nb, int sms, bool may_cluster, int32_t out[6]) {
+    const PcgSplit p = pcg_split(nslices, total_slots, nb, sms, may_cluster);
+    const int warps = (nb == 3 ? grid_threads<3>() : grid_threads<1>()) / 32;
+    int top = -1;
+    if (p.ks > 1)
+        for (int w = 0; w < warps; ++w)
+            if (warp_role(w, p.ks, warps).leader) top = 32 * (w + p.ks - 1) + 31;
+    out[0] = p.grid;
+    out[1] = p.per_cta;
+    out[2] = p.ks;
+    out[3] = p.turns;
+    out[4] = p.smem_bytes > 0;
+    out[5] = top;
+}
+
 // Runs the iterations from the state that k_pcg_start left (r, z, p = z, the scalars) until the scalars
 // say done; *gave_up is set when a launch gave up.  p2 is the second direction buffer.
 int pcg_grid(plato_problem* h, int nb, const double* vals, const double* dinv, double* x, double* p2, int32_t max_it,
@@ -282,26 +335,15 @@ int pcg_grid(plato_problem* h, int nb, const double* vals, const double* dinv, d
     int sms = 0, coop = 0;
     PLATO_CUDA(h, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
     PLATO_CUDA(h, cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h->device));
-    const int warps = (nb == 3 ? grid_threads<3>() : grid_threads<1>()) / 32;
-    const int64_t room = kGridSmemMax - (nb == 3 ? 512 * 24 : 1024 * 8) - 2048;
-    // shared memory for the average CTA's slots and a tenth more; a CTA with more reads L2
-    const auto smem_for = [&](int ctas) { return (h->sell.total_slots / ctas + 32) * (8 * nb * nb + 4) * 11 / 10; };
-    // A system that gives each of 16 SMs its part in shared memory and each slice 3 warps (scalar: one) runs
-    // as one cluster, whose barrier is a hardware one.  One grid-wide counter against this: 12x6x6 2.0 -> 1.4 ms,
-    // 18x9x9 3.0 -> 2.3, 20x10x10 (80 slices, 3 warps each) 3.2 -> 2.5; with 2 warps a slice 21x10x10 3.38 -> 3.41,
-    // so the line lies there.  Filter: 16x8x8 0.49 -> 0.38 ms, 37x20x18 (474 slices, a warp each) 0.97 -> 0.86.
-    int cluster = 1;
-    while (2 * cluster <= std::min<int>(kClusterMax, h->sell.nslices)) cluster *= 2;
-    int clustered = (h->sell.nslices + cluster - 1) / cluster * (nb == 3 ? 3 : 1) <= warps && smem_for(cluster) <= room;
-    int grid = clustered ? cluster : std::min({sms, h->sell.nslices, 32 * warps});
-    int per_cta = (h->sell.nslices + grid - 1) / grid;
-    if (!coop || per_cta > 2 * warps || (nb == 3 && per_cta > warps)) {
+    const bool slices_fit = pcg_split(h->sell.nslices, h->sell.total_slots, nb, sms, false).turns <= (nb == 3 ? 1 : 2);
+    if (!coop || !slices_fit) {
         PLATO_CUDA(h, cudaMemcpyAsync(h->scal_host, h->scal, sizeof(PcgScalars), cudaMemcpyDeviceToHost, h->stream));
         PLATO_CUDA(h, cudaStreamSynchronize(h->stream));
         *fin = h->scal_host[0];
         *gave_up = 1;
         return PLATO_OK;
     }
+    PcgSplit split = pcg_split(h->sell.nslices, h->sell.total_slots, nb, sms, true);
     GridPcg a{};
     a.A = sell_view(h);
     a.nslices = h->sell.nslices;
@@ -315,21 +357,20 @@ int pcg_grid(plato_problem* h, int nb, const double* vals, const double* dinv, d
     a.max_it = max_it;
     a.S = h->scal;
     for (;;) {
-        a.ks = std::max(1, warps / per_cta);
-        const int64_t want = smem_for(grid);
-        a.smem_bytes = want <= room ? int((want + 15) / 16 * 16) : 0;
+        a.ks = split.ks;
+        a.smem_bytes = int(split.smem_bytes);
         PLATO_RC(grid_box(h, &a.box));
-        if (clustered) {
-            if (nb == 3) PLATO_RC(launch_cluster<3>(h, a, grid, &clustered));
-            else PLATO_RC(launch_cluster<1>(h, a, grid, &clustered));
-            if (!clustered) {
-                grid = std::min({sms, h->sell.nslices, 32 * warps});
-                per_cta = (h->sell.nslices + grid - 1) / grid;
+        if (split.clustered) {
+            int ok = 1;
+            if (nb == 3) PLATO_RC(launch_cluster<3>(h, a, split.grid, &ok));
+            else PLATO_RC(launch_cluster<1>(h, a, split.grid, &ok));
+            if (!ok) {
+                split = pcg_split(h->sell.nslices, h->sell.total_slots, nb, sms, false);
                 continue;
             }
-        } else if (nb == 3) PLATO_RC((launch_grid<3, 1>(h, a, grid)));
-        else if (per_cta <= warps) PLATO_RC((launch_grid<1, 1>(h, a, grid)));
-        else PLATO_RC((launch_grid<1, 2>(h, a, grid)));
+        } else if (nb == 3) PLATO_RC((launch_grid<3, 1>(h, a, split.grid)));
+        else if (split.turns == 1) PLATO_RC((launch_grid<1, 1>(h, a, split.grid)));
+        else PLATO_RC((launch_grid<1, 2>(h, a, split.grid)));
         int32_t abort = 0;
         PLATO_CUDA(h, cudaMemcpyAsync(h->scal_host, h->scal, sizeof(PcgScalars), cudaMemcpyDeviceToHost, h->stream));
         PLATO_CUDA(h, cudaMemcpyAsync(&abort, a.box.abort, sizeof(abort), cudaMemcpyDeviceToHost, h->stream));

@@ -12,7 +12,7 @@ from helpers import rel_l2
 from oracle import Oracle
 from platoanalyze_b200 import capi
 from platoanalyze_b200.mesh import box_mesh
-from platoanalyze_b200.problem import EllipticProblem, HelmholtzFilter, SolverOptions
+from platoanalyze_b200.problem import EllipticProblem, HelmholtzFilter, ProblemSpec, SolverOptions
 from platoanalyze_b200.workloads import cantilever, coarse_grid, method_options, splitmix_uniform
 
 pytestmark = pytest.mark.gpu
@@ -142,3 +142,74 @@ def test_sweep_on_both_sides_of_the_l2(size):
         assert st["converged"] and st["fallback"] == 0 and st["relative_residual"] <= 1e-10, st
         got.append(u.cpu().numpy())
     assert rel_l2(*got) <= 1e-8
+
+
+def _split(p, nb):
+    out = np.zeros(6, np.int32)
+    slices = (p.num_nodes + 31) // 32
+    assert capi.lib.plato_test_pcg_split(slices, p.sell_info()["total_slots"], nb, 148, 1, out.ctypes.data_as(capi.i32p)) == capi.OK
+    return {"per_cta": int(out[1]), "parts": int(out[2]), "in_smem": int(out[4])}
+
+
+@pytest.mark.parametrize("size,per_cta,parts", [((13, 9, 9), 3, 5), ((20, 10, 10), 5, 3), ((40, 18, 16), 3, 5), ((48, 21, 20), 5, 3)],
+                         ids=str)
+def test_shares_that_leave_warps_over(size, per_cta, parts):
+    """3 and 5 slices on the 16 warps of a CTA: 5 and 3 warps each and one left over, as a cluster and as a
+    grid.  The bars of the other comparisons with the launch per stage."""
+    spec = cantilever(*size, method_options("plain", 1e-10, (2, 1, 1)))
+    z = splitmix_uniform(spec.coords.shape[0], 3, 0.2, 1.0)
+    p = EllipticProblem(spec)
+    assert _split(p, 3) == {"per_cta": per_cta, "parts": parts, "in_smem": 1}
+    u, st = p.solution(p.to_dev(z))
+    p.set_timing(True)
+    v, sv = p.solution(p.to_dev(z))
+    assert st["converged"] and sv["converged"] and abs(st["iterations"] - sv["iterations"]) <= max(3, sv["iterations"] // 20)
+    assert rel_l2(u.cpu().numpy(), v.cpu().numpy()) <= 1e-8
+
+
+def mirrored_box(nx, ny, nz):
+    """A box whose hexes are cut like the mirror images of their neighbours: the cells of box_mesh's shape, but
+    every other node has 26 neighbours, so that nearly every slice of 32 rows is 27 blocks wide."""
+    m = box_mesh(nx, ny, nz, 2.0, 1.0, 1.0)
+    n = np.array([nx + 1, ny + 1, nz + 1])
+    at = np.stack(np.unravel_index(m.connectivity, n), -1)  # the cells of a hex are 6 in a row
+    low = at.reshape(-1, 24, 3).min(1)[:, None, None, :]
+    offset = (at.reshape(-1, 6, 4, 3) - low) ^ (low & 1)
+    return m, np.ascontiguousarray(np.ravel_multi_index(tuple(np.moveaxis(low + offset, -1, 0)), n).reshape(-1, 4), np.int32)
+
+
+def test_shares_that_leave_warps_over_from_l2():
+    """5 slices a CTA with rows so wide that the matrix does not fit in shared memory."""
+    m, conn = mirrored_box(48, 21, 20)
+    fixed = np.nonzero(m.coords[:, 0] == 0.0)[0]
+    dofs = (3 * fixed[:, None] + np.arange(3)).reshape(-1).astype(np.int32)
+    on = m.coords[conn, 0] == 2.0
+    cells = np.nonzero(on.sum(1) == 3)[0]
+    local = np.nonzero(on[cells])[1].reshape(-1, 3)
+    spec = ProblemSpec(m.coords, conn, 1.0, 0.3, 3.0, 1e-9, [(cells.astype(np.int32), local.astype(np.int32), (0.0, -1.0, 0.0))],
+                       dofs, np.zeros(dofs.size), method_options("plain", 1e-10, (2, 1, 1)))
+    z = splitmix_uniform(m.num_nodes, 3, 0.2, 1.0)
+    p = EllipticProblem(spec)
+    assert _split(p, 3) == {"per_cta": 5, "parts": 3, "in_smem": 0}
+    u, st = p.solution(p.to_dev(z))
+    p.set_timing(True)
+    w, sw = p.solution(p.to_dev(z))
+    assert st["converged"] and sw["converged"] and abs(st["iterations"] - sw["iterations"]) <= max(3, sw["iterations"] // 20)
+    assert rel_l2(u.cpu().numpy(), w.cpu().numpy()) <= 1e-8
+
+
+@pytest.mark.parametrize("size,per_cta", [((13, 9, 9), 3), ((18, 11, 10), 5), ((20, 11, 11), 6), ((24, 14, 11), 9),
+                                          ((48, 21, 20), 5), ((50, 22, 20), 6), ((60, 26, 24), 9), ((62, 26, 25), 10)], ids=str)
+def test_filter_shares_that_leave_warps_over(size, per_cta):
+    """The scalar systems with 3 to 10 slices on the 32 warps of a CTA, as a cluster and as a grid."""
+    m = box_mesh(*size, 2.0, 1.0, 1.0)
+    f = HelmholtzFilter(m.coords, m.connectivity, 0.08)
+    slices = (m.num_nodes + 31) // 32
+    out = np.zeros(6, np.int32)
+    assert capi.lib.plato_test_pcg_split(slices, 15 * 32 * slices, 1, 148, 1, out.ctypes.data_as(capi.i32p)) == capi.OK
+    assert out[1] == per_cta and 32 % out[2] != 0
+    c = f.to_dev(splitmix_uniform(m.num_nodes, 4))
+    a, sa = f.solution(c)
+    f.set_timing(True)
+    b, sb = f.solution(c)
+    assert abs(sa["iterations"] - sb["iterations"]) <= 2 and rel_l2(a.cpu().numpy(), b.cpu().numpy()) <= 1e-10
