@@ -214,6 +214,12 @@ int plato_get_sweep_info(const plato_problem* h, int32_t* steps_per_launch, int3
  * the solve reports the timeout to the host, the multi-step sweep is switched off for the
  * handle and the plain FP64 Jacobi-PCG fallback finishes the solve (fallback_max_iterations). */
 int plato_test_stall_next_sweep(plato_problem* h);
+/* Test hook for the bounded waits of the cooperative Krylov loops (no reference counterpart): in the next
+ * such launch of this handle (one that is not a single cluster) the wait of CTA `cta` at its barrier number
+ * `barrier` (from 1) runs out after some ten milliseconds; with iterations > 0 a flexible-CG launch ends
+ * after that many iterations, so that its last barrier can be met.  All CTAs leave, and the solve goes on from the x
+ * that is there with one launch per stage, as does every later solve of the handle. */
+int plato_test_stall_next_grid(plato_problem* h, int32_t cta, int32_t barrier, int32_t iterations);
 /* Test hook (no reference counterpart): how the cooperative Jacobi-PCG lays a system of nslices slices of
  * 32 rows, total_slots slots in all, over `sms` SMs (without a device): out = {CTAs, slices of the largest
  * share, warps per slice, slices a group of warps takes in turn, 1 if the matrix is kept in shared

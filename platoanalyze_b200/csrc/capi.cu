@@ -457,6 +457,12 @@ int plato_test_stall_next_sweep(plato_problem* h) {
     return PLATO_OK;
 }
 
+int plato_test_stall_next_grid(plato_problem* h, int32_t cta, int32_t barrier, int32_t iterations) {
+    if (!h || cta < 0 || barrier < 1 || iterations < 0) return PLATO_BAD_INPUT;
+    h->grid_stall = GridStall{cta, uint32_t(barrier), iterations};
+    return PLATO_OK;
+}
+
 int plato_test_pcg_split(int32_t nslices, int64_t total_slots, int32_t unknowns_per_row, int32_t sms, int32_t may_cluster,
                          int32_t out[6]) {
     if (!out || nslices < 1 || total_slots < 32 || sms < 1 || (unknowns_per_row != 1 && unknowns_per_row != 3))

@@ -189,7 +189,12 @@ __global__ void __launch_bounds__(kGridThreads, 1) k_fcg_grid(const __grid_const
     __shared__ double sh_cta[kGridValues][32], sh_grid[kGridValues][32];
     __shared__ double part[3][kGridThreads];
     int32_t done = a.S->done;
-    if (done || *reinterpret_cast<volatile int32_t*>(a.box.abort)) return;
+    if (done || *reinterpret_cast<volatile int32_t*>(a.box.abort)) {
+        // an abort that CTA 0 did not see in its own launch (another CTA's wait ran out at the last barrier) ends
+        // the host's loop here: it looks at done
+        if (!done && blockIdx.x == 0 && threadIdx.x == 0) a.S->done = 1;
+        return;
+    }
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int s0 = int((int64_t)a.nslices * blockIdx.x / gridDim.x), s1 = int((int64_t)a.nslices * (blockIdx.x + 1) / gridDim.x);
     const int kg = warp % a.ks, s = s0 + warp / a.ks;
@@ -418,7 +423,7 @@ int fcg_grid_iterations(plato_problem* h, int entry_bytes, bool half_entries, co
     a.degree = degree;
     a.coarse = coarse;
     a.max_it = max_it;
-    a.iters = kLaunchIters;
+    a.iters = h->grid_stall.iterations > 0 ? h->grid_stall.iterations : kLaunchIters;
     a.S = h->scal;
     a.cc = cc;
     if (coarse) {
@@ -450,7 +455,7 @@ int fcg_grid_iterations(plato_problem* h, int entry_bytes, bool half_entries, co
 
 int fcg_grid_gave_up(plato_problem* h, int* gave_up) {
     GridBox m;
-    PLATO_RC(grid_box(h, &m));
+    PLATO_RC(grid_box(h, &m));  // (no stall is pending: the loop's first launch has taken it)
     int32_t abort = 0;
     PLATO_CUDA(h, cudaMemcpyAsync(&abort, m.abort, sizeof(abort), cudaMemcpyDeviceToHost, h->stream));
     PLATO_CUDA(h, cudaStreamSynchronize(h->stream));

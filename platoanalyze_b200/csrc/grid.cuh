@@ -21,6 +21,9 @@ struct GridBox {
     double*   box;    // [2][kGridValues][gridDim.x]
     uint32_t* count;  // arrivals in this launch
     int32_t*  abort;
+    uint32_t  polls;  // limit of a wait
+    int32_t   stall_cta;      // test hook: this CTA's wait at this barrier is for arrivals that never come
+    uint32_t  stall_barrier;  // (0: none)
 };
 
 // acquire-release at GPU scope; __threadfence() is the sequentially consistent one, which costs more
@@ -28,13 +31,14 @@ __device__ __forceinline__ void grid_fence() { asm volatile("fence.acq_rel.gpu;"
 
 // Thread 0 of a CTA whose other threads' writes a __syncthreads() has put before this.
 __device__ __forceinline__ bool grid_arrive_and_wait(const GridBox& a, uint32_t barrier) {
-    const uint32_t target = barrier * gridDim.x;
+    const bool stalled = barrier == a.stall_barrier && int(blockIdx.x) == a.stall_cta;
+    const uint32_t target = barrier * gridDim.x + (stalled ? 1u << 30 : 0u);
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.count) : "memory");
     for (uint32_t polls = 1;; ++polls) {
         uint32_t v;
         asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.count) : "memory");
         if (int32_t(v - target) >= 0) break;
-        if (polls > kGridPolls || ((polls & 1023u) == 0 && *reinterpret_cast<volatile int32_t*>(a.abort))) {
+        if (polls > a.polls || ((polls & 1023u) == 0 && *reinterpret_cast<volatile int32_t*>(a.abort))) {
             *reinterpret_cast<volatile int32_t*>(a.abort) = 1;
             return false;
         }
@@ -162,7 +166,8 @@ __host__ __device__ __forceinline__ WarpRole warp_role(int warp, int parts, int 
     return {part, group, part == 0 && group < warps / parts};
 }
 
-// The boxes, counter (cleared for the next launch) and abort flag of a handle (pcg_grid.cu).
+// The boxes, counter and abort flag of a handle for its next launch: the counter is cleared, and a stall that the
+// test hook asked for is taken up (pcg_grid.cu).
 int grid_box(plato_problem* h, GridBox* box);
 
 }  // namespace plato

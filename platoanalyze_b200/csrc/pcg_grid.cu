@@ -16,6 +16,7 @@
 // 1.92 -> 0.96, 100x50x50 3.30 -> 1.69, 112x53x52 (the largest that qualifies) 4.00 -> 3.81: there the
 // CTAs read the matrix from L2 with two slices per warp, hence the limits in pcg_grid_ok.
 #include <algorithm>
+#include <utility>
 
 #include "grid.cuh"
 #include "plato_internal.cuh"
@@ -263,6 +264,10 @@ int grid_box(plato_problem* h, GridBox* box) {
     box->abort = reinterpret_cast<int32_t*>(static_cast<char*>(h->grid_box) + 64);
     box->box = reinterpret_cast<double*>(static_cast<char*>(h->grid_box) + 128);
     PLATO_CUDA(h, cudaMemsetAsync(box->count, 0, sizeof(uint32_t), h->stream));
+    const GridStall stall = std::exchange(h->grid_stall, GridStall{});
+    box->polls = stall.barrier ? kGridPolls >> 6 : kGridPolls;
+    box->stall_cta = stall.cta;
+    box->stall_barrier = stall.barrier;
     return PLATO_OK;
 }
 

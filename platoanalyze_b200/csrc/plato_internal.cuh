@@ -155,6 +155,14 @@ struct FanPlan {
     float*    w32 = nullptr;   // the same in FP32
 };
 
+// Test hook of the cooperative Krylov loops (grid.cuh): in the next launch the wait of CTA `cta` at barrier `barrier`
+// runs out; a flexible-CG launch ends after `iterations`, when that is not 0.
+struct GridStall {
+    int32_t  cta = -1;
+    uint32_t barrier = 0;
+    int32_t  iterations = 0;
+};
+
 // Two-level preconditioner state (coarse.cu).
 struct CoarseSpace {
     int      nc[3] = {0, 0, 0};   // coarse cells per axis
@@ -252,6 +260,7 @@ struct plato_problem {
     PcgScalars* scal = nullptr;    // device
     PcgScalars* scal_host = nullptr;  // pinned mirror
     void*    grid_box = nullptr;   // counter, abort flag and boxes of the cooperative Krylov loops (grid.cuh)
+    GridStall grid_stall{};
     int      grid_off = 0;         // one of its waits ran out on this handle: one launch per stage from then on
     double* red_out = nullptr;     // device scalar result of a reduction
     uint32_t* red_ticket = nullptr;

@@ -213,3 +213,43 @@ def test_filter_shares_that_leave_warps_over(size, per_cta):
     f.set_timing(True)
     b, sb = f.solution(c)
     assert abs(sa["iterations"] - sb["iterations"]) <= 2 and rel_l2(a.cpu().numpy(), b.cpu().numpy()) <= 1e-10
+
+
+# (method, size, CTA whose wait runs out, barrier, iterations of the launch).  Flexible CG of degree d: barriers 1 and 2
+# are sums, d - 2 more (with a coarse space d - 1) belong to the sweep, 5 to the coarse solve, the last two are sums.
+STALLS = [("plain", (30, 16, 16), 0, 1, 0), ("plain", (30, 16, 16), 3, 7, 0), ("plain", (40, 20, 20), 147, 40, 0),
+          ("chebyshev", (20, 10, 10), 0, 3, 0), ("chebyshev", (20, 10, 10), 1, 10, 1), ("bf16", (26, 12, 12), 5, 18, 1),
+          ("two-level", (20, 10, 10), 2, 14, 0), ("two-level-fp16", (40, 20, 20), 7, 22, 1), ("two-level-fp16", (40, 20, 20), 0, 22, 1)]
+
+
+@pytest.mark.parametrize("method,size,cta,barrier,iterations", STALLS, ids=str)
+def test_a_wait_that_runs_out(method, size, cta, barrier, iterations):
+    """A wait that runs out, in the middle of an iteration or at the last barrier of a launch, ends the launch; the
+    solve goes on with one launch per stage and meets its tolerance, and so do the handle's later solves."""
+    spec = cantilever(*size, method_options(method, 1e-10, coarse_grid(*size)))
+    z = splitmix_uniform(spec.coords.shape[0], 3, 0.2, 1.0)
+    p = EllipticProblem(spec)
+    zd = p.to_dev(z)
+    v, _ = p.solution(zd)
+    p.reset_instrumentation()
+    _, sv = p.solution(zd)
+    few = p.instrumentation()["launches"]
+    assert capi.lib.plato_test_stall_next_grid(p.h, cta, barrier, iterations) == capi.OK
+    for _ in range(2):
+        p.reset_instrumentation()
+        u, st = p.solution(zd)
+        assert st["converged"] and st["fallback"] == 0 and st["relative_residual"] <= 1e-10, st
+        assert p.instrumentation()["launches"] > few + st["iterations"]
+        assert rel_l2(u.cpu().numpy(), v.cpu().numpy()) <= 1e-8
+    assert st["iterations"] > 1 and sv["iterations"] > 1
+
+
+def test_a_wait_that_runs_out_in_the_filter():
+    m = box_mesh(48, 21, 20, 2.0, 1.0, 1.0)
+    f = HelmholtzFilter(m.coords, m.connectivity, 0.08)
+    c = f.to_dev(splitmix_uniform(m.num_nodes, 4))
+    a, _ = f.solution(c)
+    assert capi.lib.plato_test_stall_next_grid(f.h, 9, 6, 0) == capi.OK
+    for _ in range(2):
+        b, _ = f.solution(c)
+        assert rel_l2(a.cpu().numpy(), b.cpu().numpy()) <= 1e-10
