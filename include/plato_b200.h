@@ -220,6 +220,9 @@ int plato_test_stall_next_sweep(plato_problem* h);
  * after that many iterations, so that its last barrier can be met.  All CTAs leave, and the solve goes on from the x
  * that is there with one launch per stage, as does every later solve of the handle. */
 int plato_test_stall_next_grid(plato_problem* h, int32_t cta, int32_t barrier, int32_t iterations);
+/* Test hook (no reference counterpart): from now on the cooperative Krylov loops of this handle take `sms` SMs, at
+ * most those they have (0: none, one launch per stage), and the systems that fit on those. */
+int plato_test_grid_sms(plato_problem* h, int32_t sms);
 /* Test hook (no reference counterpart): how the cooperative Jacobi-PCG lays a system of nslices slices of
  * 32 rows, total_slots slots in all, over `sms` SMs (without a device): out = {CTAs, slices of the largest
  * share, warps per slice, slices a group of warps takes in turn, 1 if the matrix is kept in shared

@@ -114,6 +114,7 @@ def _load() -> C.CDLL:
         "plato_get_sweep_info": ([vp, C.POINTER(C.c_int32), C.POINTER(C.c_int32)], C.c_int),
         "plato_test_stall_next_sweep": ([vp], C.c_int),
         "plato_test_stall_next_grid": ([vp, C.c_int32, C.c_int32, C.c_int32], C.c_int),
+        "plato_test_grid_sms": ([vp, C.c_int32], C.c_int),
         "plato_test_pcg_split": ([C.c_int32, C.c_int64, C.c_int32, C.c_int32, C.c_int32, i32p], C.c_int),
         "plato_get_sizes": ([vp, i32p, i32p, C.POINTER(C.c_int64)], C.c_int),
         "plato_jacobian_pattern": ([vp, vp, vp], C.c_int),

@@ -241,6 +241,10 @@ static int create_handle(const plato_problem_desc* d, plato_problem** out) {
         }
     if (int rc = check_opts(h, h->opts)) { g_create_error = h->last_error; delete h; return rc; }
     cudaGetDevice(&h->device);
+    int coop = 0;
+    if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h->device) != cudaSuccess || !coop ||
+        cudaDeviceGetAttribute(&h->coop_sms, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess)
+        h->coop_sms = 0;
 
     // IsotropicLinearElasticMaterial<3> constants, src/IsotropicLinearElasticMaterial.cpp:86-110
     const double coef = E / ((1.0 + nu) * (1.0 - 2.0 * nu));
@@ -460,6 +464,12 @@ int plato_test_stall_next_sweep(plato_problem* h) {
 int plato_test_stall_next_grid(plato_problem* h, int32_t cta, int32_t barrier, int32_t iterations) {
     if (!h || cta < 0 || barrier < 1 || iterations < 0) return PLATO_BAD_INPUT;
     h->grid_stall = GridStall{cta, uint32_t(barrier), iterations};
+    return PLATO_OK;
+}
+
+int plato_test_grid_sms(plato_problem* h, int32_t sms) {
+    if (!h || sms < 0 || sms > h->coop_sms) return PLATO_BAD_INPUT;
+    h->coop_sms = sms;
     return PLATO_OK;
 }
 

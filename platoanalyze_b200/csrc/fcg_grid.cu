@@ -395,16 +395,13 @@ int launch(plato_problem* h, const GridFcg& a, int grid) {
 }  // namespace
 
 bool fcg_grid_ok(const plato_problem* h) {
-    return !h->grid_off && !h->timing && !h->ritz_deflating && h->sell.nslices <= int64_t(kNumSMs) * kGridWarps;
+    return !h->grid_off && !h->timing && !h->ritz_deflating && h->sell.nslices <= int64_t(h->coop_sms) * kGridWarps;
 }
 
 int fcg_grid_iterations(plato_problem* h, int entry_bytes, bool half_entries, const void* vin, const ChebCoef& cc, int degree,
                         int coarse, double* x, const float* scale, int32_t max_it) {
-    int sms = 0;
-    PLATO_CUDA(h, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
-    const int grid = std::min(sms, h->sell.nslices);
-    const int per_cta = (h->sell.nslices + grid - 1) / grid;
-    if (per_cta > kGridWarps) return plato_fail(h, PLATO_BAD_INPUT, "system too large for the cooperative iteration");
+    const int grid = std::min(h->coop_sms, h->sell.nslices);
+    const int per_cta = (h->sell.nslices + grid - 1) / grid;  // at most kGridWarps (fcg_grid_ok)
     GridFcg a{};
     a.A = sell_view(h);
     a.nslices = h->sell.nslices;

@@ -12,7 +12,7 @@ struct ChebCoef {
     float c2[64];
 };
 
-// Whether this system's iterations can run in cooperative launches: every slice has a warp, nothing
+// Whether this system's iterations can run in cooperative launches: the device has them, every slice has a warp, nothing
 // wants a look between the stages (sampled timings, deflation), and no earlier launch gave up.
 bool fcg_grid_ok(const plato_problem* h);
 

@@ -253,9 +253,7 @@ int launch_cluster(plato_problem* h, GridPcg& a, int grid, int* ok) {
 }  // namespace
 
 int grid_box(plato_problem* h, GridBox* box) {
-    int sms = 0;
-    PLATO_CUDA(h, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
-    const size_t bytes = sizeof(double) * 2 * kGridValues * size_t(sms);
+    const size_t bytes = sizeof(double) * 2 * kGridValues * size_t(h->coop_sms);
     if (!h->grid_box) {
         PLATO_CUDA(h, cudaMalloc(&h->grid_box, bytes + 128));
         PLATO_CUDA(h, cudaMemsetAsync(h->grid_box, 0, bytes + 128, h->stream));
@@ -271,13 +269,13 @@ int grid_box(plato_problem* h, GridBox* box) {
     return PLATO_OK;
 }
 
-// Whether the iterations of this system run in cooperative launches: every slice has a group of
-// warps (one slice a group for block systems, at most two for scalar ones), nothing else wants a
+// Whether the iterations of this system run in cooperative launches: the device has them, every slice has a
+// group of warps (one slice a group for block systems, at most two for scalar ones), nothing else wants a
 // look between iterations (sampled timings, a deflated direction), and no earlier launch gave up.
 bool pcg_grid_ok(const plato_problem* h, int nb) {
     if (h->grid_off || h->timing || h->ritz_deflating) return false;
     const int64_t warps = (nb == 3 ? grid_threads<3>() : grid_threads<1>()) / 32;
-    return h->sell.nslices <= int64_t(kNumSMs) * warps * (nb == 3 ? 1 : 2);
+    return h->sell.nslices <= int64_t(h->coop_sms) * warps * (nb == 3 ? 1 : 2);
 }
 
 namespace {
@@ -337,18 +335,7 @@ void pcg_split_info(int nslices, int64_t total_slots, int nb, int sms, bool may_
 int pcg_grid(plato_problem* h, int nb, const double* vals, const double* dinv, double* x, double* p2, int32_t max_it,
              PcgScalars* fin, int* gave_up) {
     *gave_up = 0;
-    int sms = 0, coop = 0;
-    PLATO_CUDA(h, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
-    PLATO_CUDA(h, cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h->device));
-    const bool slices_fit = pcg_split(h->sell.nslices, h->sell.total_slots, nb, sms, false).turns <= (nb == 3 ? 1 : 2);
-    if (!coop || !slices_fit) {
-        PLATO_CUDA(h, cudaMemcpyAsync(h->scal_host, h->scal, sizeof(PcgScalars), cudaMemcpyDeviceToHost, h->stream));
-        PLATO_CUDA(h, cudaStreamSynchronize(h->stream));
-        *fin = h->scal_host[0];
-        *gave_up = 1;
-        return PLATO_OK;
-    }
-    PcgSplit split = pcg_split(h->sell.nslices, h->sell.total_slots, nb, sms, true);
+    PcgSplit split = pcg_split(h->sell.nslices, h->sell.total_slots, nb, h->coop_sms, true);
     GridPcg a{};
     a.A = sell_view(h);
     a.nslices = h->sell.nslices;
@@ -370,7 +357,7 @@ int pcg_grid(plato_problem* h, int nb, const double* vals, const double* dinv, d
             if (nb == 3) PLATO_RC(launch_cluster<3>(h, a, split.grid, &ok));
             else PLATO_RC(launch_cluster<1>(h, a, split.grid, &ok));
             if (!ok) {
-                split = pcg_split(h->sell.nslices, h->sell.total_slots, nb, sms, false);
+                split = pcg_split(h->sell.nslices, h->sell.total_slots, nb, h->coop_sms, false);
                 continue;
             }
         } else if (nb == 3) PLATO_RC((launch_grid<3, 1>(h, a, split.grid)));

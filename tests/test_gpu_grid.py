@@ -253,3 +253,23 @@ def test_a_wait_that_runs_out_in_the_filter():
     for _ in range(2):
         b, _ = f.solution(c)
         assert rel_l2(a.cpu().numpy(), b.cpu().numpy()) <= 1e-10
+
+
+@pytest.mark.parametrize("sms", [5, 4, 0])
+@pytest.mark.parametrize("method", ["plain", "chebyshev", "two-level-fp16"])
+def test_a_device_with_fewer_sms(method, sms):
+    """80 slices on 5 SMs, the most that 16 warps each hold, on 4, which are too few, and on a device without
+    cooperative launches: the same solution, by the launch per stage in the last two."""
+    spec = cantilever(20, 10, 10, method_options(method, 1e-10, (2, 1, 1)))
+    p = EllipticProblem(spec)
+    zd = p.to_dev(splitmix_uniform(p.num_nodes, 3, 0.2, 1.0))
+    p.solution(zd)
+    p.reset_instrumentation()
+    v, _ = p.solution(zd)
+    few = p.instrumentation()["launches"]
+    assert capi.lib.plato_test_grid_sms(p.h, sms) == capi.OK and capi.lib.plato_test_grid_sms(p.h, sms + 1) == capi.BAD_INPUT
+    p.reset_instrumentation()
+    u, st = p.solution(zd)
+    assert st["converged"] and st["fallback"] == 0 and st["relative_residual"] <= 1e-10, st
+    assert (p.instrumentation()["launches"] > few + st["iterations"]) == (sms < 5)
+    assert rel_l2(u.cpu().numpy(), v.cpu().numpy()) <= 1e-8
