@@ -129,7 +129,8 @@ typedef struct plato_solver_opts {
                                  for the tiles of the step before that its columns reach, so the
                                  matrix can be re-read from L2 (needs 16-bit column offsets).
                                  Systems of up to some 75,000 nodes run their iterations in
-                                 cooperative launches instead, whatever this says             */
+                                 cooperative launches instead, whatever this says, and sweep so
+                                 only once per solve (plato_get_loop_info tells)              */
     int32_t sweep_lag;        /* multi-step sweep: tiles of 512 rows by which each step trails the
                                  one before beyond the column reach (0 = 600 / sweep_steps)  */
 } plato_solver_opts;
@@ -208,6 +209,11 @@ int plato_get_kernel_timing(const plato_problem* h, int32_t kind, double* ms_tot
  * per step; > 1 = the multi-step sweep) and its column reach in tiles of 512 rows (-1 when
  * not measured). */
 int plato_get_sweep_info(const plato_problem* h, int32_t* steps_per_launch, int32_t* halo_tiles);
+/* The loop of the last solve: 1 when its iterations ran in cooperative launches, hundreds in one (every step of
+ * every sweep inside; the steps per launch above are then those of the first preconditioner application
+ * only), 0 when they ran with one launch per stage.  A batch and the matrix-free operator always do the latter, and so
+ * does a solve with sampled timings on. */
+int plato_get_loop_info(const plato_problem* h, int32_t* cooperative);
 /* Test hook for the bounded device waits (no reference counterpart): the next multi-step sweep
  * launch of this handle waits for a completion stamp that none of its tasks writes, so its
  * first dependency wait gives up after its poll limit (about a second).  The launch then ends,

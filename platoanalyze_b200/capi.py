@@ -112,6 +112,7 @@ def _load() -> C.CDLL:
         "plato_get_kernel_timing": ([vp, C.c_int32, f64p, C.POINTER(C.c_int64)], C.c_int),
         "plato_get_sell_info": ([vp, C.POINTER(C.c_int64), C.POINTER(C.c_int32)], C.c_int),
         "plato_get_sweep_info": ([vp, C.POINTER(C.c_int32), C.POINTER(C.c_int32)], C.c_int),
+        "plato_get_loop_info": ([vp, i32p], C.c_int),
         "plato_test_stall_next_sweep": ([vp], C.c_int),
         "plato_test_stall_next_grid": ([vp, C.c_int32, C.c_int32, C.c_int32], C.c_int),
         "plato_test_grid_sms": ([vp, C.c_int32], C.c_int),

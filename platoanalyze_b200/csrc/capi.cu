@@ -488,6 +488,12 @@ int plato_get_sweep_info(const plato_problem* h, int32_t* steps_per_launch, int3
     return PLATO_OK;
 }
 
+int plato_get_loop_info(const plato_problem* h, int32_t* cooperative) {
+    if (!h || !cooperative) return PLATO_BAD_INPUT;
+    *cooperative = h->grid_used;
+    return PLATO_OK;
+}
+
 int plato_get_sell_info(const plato_problem* h, int64_t* total_slots, int32_t* column_bytes) {
     if (!h || !total_slots || !column_bytes) return PLATO_BAD_INPUT;
     *total_slots = h->sell.total_slots;

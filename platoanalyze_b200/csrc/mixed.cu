@@ -1369,6 +1369,7 @@ int fcg_poly(plato_problem* h, const double* b, double* x, plato_solve_stats* st
         // systems that fit run their iterations in cooperative launches, hundreds in one, whatever
         // sweep_steps says (every step of every sweep is in the launch)
         const bool grid = !mf && !h->wave_stall && fcg_grid_ok(h);
+        h->grid_used = grid;
         int32_t chunk = grid ? 1 : kChunk;
         for (;;) {
             for (int k = 0; k < chunk; ++k, ++enqueued) {
@@ -1825,6 +1826,7 @@ int fcg_batch(plato_problem* h, const double* b, double* x, plato_solve_stats* s
     const int kind = inner_kind(h);
     if (kind == INNER_SELL16S)
         return plato_fail(h, PLATO_NOT_SUPPORTED, "the FP16 scaled inner precision is built for single problems");
+    h->grid_used = 0;
     const SellView V = sell_view(h);
     // persistent grid: the autotuned CTAs per SM x SMs (never more CTAs than tiles), one row of
     // a tile per thread

@@ -261,6 +261,7 @@ struct plato_problem {
     PcgScalars* scal_host = nullptr;  // pinned mirror
     void*    grid_box = nullptr;   // counter, abort flag and boxes of the cooperative Krylov loops (grid.cuh)
     int      coop_sms = 0;         // SMs that a cooperative launch may use (0: the device has no such launches)
+    int      grid_used = 0;        // the last solve's iterations ran in cooperative launches
     GridStall grid_stall{};
     int      grid_off = 0;         // one of its waits ran out on this handle: one launch per stage from then on
     double* red_out = nullptr;     // device scalar result of a reduction

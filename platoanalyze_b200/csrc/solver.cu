@@ -351,6 +351,7 @@ static int pcg_run(plato_problem* h, int64_t n, int nb, const double* vals, Appl
         int32_t chunk = kChunk;
         PcgScalars fin;
         const bool grid = pcg_grid_ok(h, nb);
+        h->grid_used = grid;
         if (grid) {  // the whole loop in cooperative launches
             int gave_up = 0;
             rc = pcg_grid(h, nb, vals, dinv, x, p2 ? p2 : h->v_tmp, max_it, &fin, &gave_up);

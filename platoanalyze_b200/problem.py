@@ -204,10 +204,13 @@ class EllipticProblem:
 
     def sweep_info(self) -> dict:
         """The FP16 sweep of the last flexible-CG solve: Chebyshev steps per launch (1: one
-        launch per step) and the column reach in tiles of 512 rows (-1: not measured)."""
-        steps, halo = C.c_int32(), C.c_int32()
+        launch per step) and the column reach in tiles of 512 rows (-1: not measured); cooperative: the
+        iterations ran in cooperative launches, which have the sweeps inside, and the steps per launch are
+        those of the first preconditioner application only."""
+        steps, halo, coop = C.c_int32(), C.c_int32(), C.c_int32()
+        check(lib.plato_get_loop_info(self.h, C.byref(coop)), self.h)
         check(lib.plato_get_sweep_info(self.h, C.byref(steps), C.byref(halo)), self.h)
-        return {"steps_per_launch": steps.value, "halo_tiles": halo.value}
+        return {"steps_per_launch": steps.value, "halo_tiles": halo.value, "cooperative": bool(coop.value)}
 
     def reset_instrumentation(self) -> None:
         check(lib.plato_reset_instrumentation(self.h), self.h)

@@ -273,3 +273,30 @@ def test_a_device_with_fewer_sms(method, sms):
     assert st["converged"] and st["fallback"] == 0 and st["relative_residual"] <= 1e-10, st
     assert (p.instrumentation()["launches"] > few + st["iterations"]) == (sms < 5)
     assert rel_l2(u.cpu().numpy(), v.cpu().numpy()) <= 1e-8
+
+
+@pytest.mark.parametrize("cells", [(20, 10, 10), (40, 20, 20)], ids=str)
+def test_multistep_sweep_on_the_staged_loop(cells):
+    """The multi-step sweep in every iteration of small systems, which leave it to the cooperative loop otherwise:
+    launch lengths that do and do not divide the degree, a one-tile lag and a long one do the same arithmetic per row as one
+    launch per step, so the same iterations and the same solution (the bar of the small meshes' other test)."""
+    spec = cantilever(*cells, SolverOptions(tolerance=1e-10))
+    p = EllipticProblem(spec)
+    zd = p.to_dev(splitmix_uniform(p.num_nodes, 0x5EED0003))
+    opts = SolverOptions(tolerance=1e-10, precision=capi.PRECISION_MIXED_FP16, chebyshev_degree=9, chebyshev_ratio=100.0,
+                         coarse_cells=tuple(c // 10 for c in cells), sweep_steps=4)
+    p.set_solver(opts)
+    v, _ = p.solution(zd)
+    assert p.sweep_info()["cooperative"]
+    assert capi.lib.plato_test_grid_sms(p.h, 0) == capi.OK
+    got = []
+    for opts.sweep_steps, opts.sweep_lag in ((1, 0), (2, 0), (3, 0), (4, 0), (7, 1), (16, 0), (0, 0), (5, 300)):
+        p.set_solver(opts)
+        u, st = p.solution(zd)
+        assert st["converged"] and st["fallback"] == 0, (opts, st)
+        info = p.sweep_info()
+        assert info["steps_per_launch"] == max(1, opts.sweep_steps) and not info["cooperative"]
+        got.append((st["iterations"], u.cpu().numpy()))
+    for it, u in got[1:]:
+        assert it == got[0][0] and rel_l2(u, got[0][1]) <= 1e-14
+    assert rel_l2(v.cpu().numpy(), got[0][1]) <= 1e-8
