@@ -165,7 +165,10 @@ int plato_create(const plato_problem_desc* desc, plato_problem** out);
 int plato_destroy(plato_problem* h);
 /* Last error text of a handle (or of the last failed plato_create when h is NULL). */
 const char* plato_last_error(const plato_problem* h);
-/* Bind the handle to a CUDA stream (cudaStream_t); NULL means the legacy default stream. */
+/* Bind the handle to a CUDA stream (cudaStream_t); NULL means the legacy default stream.  The residual, the
+ * internal force, the control derivatives and the matrix-free product share scratch of the handle: such a call waits
+ * on its stream for the handle's last one on another stream.  (Not inside a stream capture: a graph that holds such a
+ * call and the handle's other calls are put in order by the caller.) */
 int plato_set_stream(plato_problem* h, void* cuda_stream);
 int plato_set_solver_opts(plato_problem* h, const plato_solver_opts* opts);
 /* Control layout (no reference counterpart: the reference's control is nodal and each cell

@@ -366,6 +366,7 @@ void fan_release(plato_problem* h) {
     FanPlan& f = h->fans;
     for (void* p : {f.mem[0], f.mem[1], (void*)f.w64, (void*)f.w32})
         if (p) cudaFree(p);
+    if (f.end) cudaEventDestroy(f.end);
     f = FanPlan{};
 }
 
@@ -527,6 +528,7 @@ int fan_plan(plato_problem* h) {
     PLATO_CUDA(h, scan<false>(mem, count, P.node_ptr, int64_t(N) + 1));
 
     PLATO_CUDA(h, cudaStreamSynchronize(s));
+    PLATO_CUDA(h, cudaEventCreateWithFlags(&P.end, cudaEventDisableTiming));
     P.nfans = nf;
     P.ntiles = nt;
     P.width = W;

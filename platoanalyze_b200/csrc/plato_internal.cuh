@@ -153,6 +153,10 @@ struct FanPlan {
     double*   sums = nullptr;  // [kFanMaxCtas] block sums of the criteria
     double*   w64 = nullptr;   // [6 * nfans] SIMP weight of each cell (matrix-free operator)
     float*    w32 = nullptr;   // the same in FP32
+    // the stream of the last call that used `part`, and its end there (fan_begin, fan_end)
+    cudaStream_t last = nullptr;
+    cudaEvent_t  end = nullptr;
+    int          pending = 0;  // 0: nothing to wait for, 1: `last` is the legacy stream, 2: `end` is recorded
 };
 
 // Test hook of the cooperative Krylov loops (grid.cuh): in the next launch the wait of CTA `cta` at barrier `barrier`
