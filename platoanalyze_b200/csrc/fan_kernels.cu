@@ -317,6 +317,81 @@ k_fans(FanView fv, Material mat, FanArgs<T> A, const PcgScalars* S) {
     }
 }
 
+// A scalar quantity cell by cell, a thread each, where the fans are short (cells_win in fans.cu): the derivative per
+// cell goes to cell_out (one density per cell) or to part, from where k_cell_nodes sums it per node.  Four CTAs an SM at 64
+// registers hide the 14 to 40 gathers of a cell, which bound it: kernels of 1.1 M Delaunay cells, dC/dz 24.7 + 17.0
+// us, (dR/dz)^T lambda 36.1 + 17.3 us (a fan with its 168 registers: 55 and 77 us together).
+constexpr int kCellThreads = 256;
+template <int OP, int MODE>
+__global__ void __launch_bounds__(kCellThreads, 4)
+k_cells(int32_t C, const int4* __restrict__ conn, const double* __restrict__ coords, Material mat, FanArgs<double> A) {
+    constexpr bool U = fan_has_u<OP>(), L = fan_has_lam<OP, MODE>();
+    constexpr bool NODES = fan_nodes<OP, MODE>(), SUMS = fan_sums<OP, MODE>();
+    double total = 0.0;
+    double* out = mat.cell_control ? A.cell_out : A.part;
+    const bool add = mat.cell_control && A.accumulate;
+    for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < C; c += (int64_t)gridDim.x * blockDim.x) {
+        const int4 n = __ldg(conn + c);
+        auto at = [](const double* v, int64_t a) { return Vec3<double>{__ldg(v + 3 * a), __ldg(v + 3 * a + 1), __ldg(v + 3 * a + 2)}; };
+        const Vec3<double> xa = at(coords, n.x);
+        const Vec3<double> eb = at(coords, n.y) - xa, ep = at(coords, n.z) - xa, en = at(coords, n.w) - xa;
+        const Vec3<double> cb = cross(ep, en), cp = cross(en, eb), cn = cross(eb, ep);
+        const double det = fabs(dot(eb, cb));
+        const double rho = cell_rho(mat, A.z, c, n);
+        double q = det * (1.0 / 6.0);  // the volume, or vol eps(u).C.eps(u) and with lambda vol eps(lambda).C.eps(u)
+        if (U) {
+            const double k = 1.0 / (6.0 * det);
+            const Vec3<double> ua = at(A.u, n.x);
+            double e[6], s[6], esl = 0.0;
+            fan_strain(at(A.u, n.y) - ua, at(A.u, n.z) - ua, at(A.u, n.w) - ua, cb, cp, cn, e);
+            stress_voigt(mat, e, s);
+            if (MODE != 3) q = k * (s[0] * e[0] + s[1] * e[1] + s[2] * e[2] + s[3] * e[3] + s[4] * e[4] + s[5] * e[5]);
+            if (L) {
+                const Vec3<double> la = at(A.lam, n.x);
+                fan_strain(at(A.lam, n.y) - la, at(A.lam, n.z) - la, at(A.lam, n.w) - la, cb, cp, cn, e);
+                esl = k * (s[0] * e[0] + s[1] * e[1] + s[2] * e[2] + s[3] * e[3] + s[4] * e[4] + s[5] * e[5]);
+            }
+            if (SUMS) total += 0.5 * q * simp(mat, rho);
+            q = MODE == 3 ? esl : 0.5 * q + esl;
+            if (MODE == 2 || MODE == 5) q = -q;
+        } else if (SUMS) {
+            total += q * simp(mat, rho);
+        }
+        if (NODES) {
+            q *= simp_dx(mat, rho) * rho_dz(mat);
+            out[c] = add ? out[c] + q : q;
+        }
+    }
+    pdl_trigger();
+    if (SUMS) {
+        __shared__ double sh[1][32];
+        __shared__ bool last;
+        double v[1] = {total};
+        block_sum_n<1>(v, sh);
+        if (publish_partials<1>(v, A.sums, A.ticket, &last)) {
+            double t[1];
+            final_sums<1>(t, A.sums, sh);
+            if (threadIdx.x == 0) {
+                *A.result = t[0];
+                *A.ticket = 0u;
+            }
+        }
+    }
+}
+
+// out[a] = sum of the quantity over the node's cells in cell order, or added to out.
+__global__ void __launch_bounds__(kThreads)
+k_cell_nodes(int32_t N, const int32_t* __restrict__ n2c_ptr, const int32_t* __restrict__ n2c, const double* __restrict__ part,
+             double* __restrict__ out, int accumulate) {
+    pdl_wait();
+    for (int64_t a = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; a < N; a += (int64_t)gridDim.x * blockDim.x) {
+        double sum = 0.0;
+        const int32_t k1 = __ldg(n2c_ptr + a + 1);
+        for (int32_t k = __ldg(n2c_ptr + a); k < k1; ++k) sum += part[__ldg(n2c + k) >> 2];
+        out[a] = accumulate ? out[a] + sum : sum;
+    }
+}
+
 // out[a] = sum of the node's tile sums in slot order, plus scale * F[a] (F != null), or added to
 // out (accumulate).  copy != null: constrained dofs take copy's value instead (identity rows).
 template <int NV, typename T>
@@ -480,6 +555,36 @@ int launch_fan_nodes(plato_problem* h, T* out, const T* F, T scale, int accumula
     return fan_end(h);
 }
 
+// A scalar quantity, by fans or by cells; with one density per node its nodal sums go to `out`, or are added to it.
+template <int OP, int MODE>
+int launch_scalar(plato_problem* h, const Material& mat, FanArgs<double> A, double* out) {
+    constexpr bool nodes = fan_nodes<OP, MODE>();
+    PLATO_RC(fan_plan(h));
+    if (!h->fans.by_cell) {
+        PLATO_RC((launch_fans<OP, MODE, double>(h, mat, A, nullptr)));
+        if (!nodes || mat.cell_control) return PLATO_OK;
+        return launch_fan_nodes<1, double>(h, out, nullptr, 0.0, A.accumulate, nullptr, nullptr);
+    }
+    PLATO_RC(fan_begin(h));
+    A.part = h->fans.part;
+    A.sums = h->fans.sums;
+    A.ticket = h->red_ticket;
+    // a sum takes one resident wave, whose last CTA then has few block sums to add (energy of 1.1 M cells 26.7 us, 36 with
+    // a CTA for every 256 cells)
+    int wave = kFanMaxCtas;
+    if (fan_sums<OP, MODE>())
+        PLATO_RC(resident_ctas(h, reinterpret_cast<const void*>(k_cells<OP, MODE>), kCellThreads, 0, &wave));
+    k_cells<OP, MODE><<<grid_for(h->C, kCellThreads, wave), kCellThreads, 0, h->stream>>>(h->C, h->conn, h->coords, mat, A);
+    PLATO_LAUNCH_CHECK(h);
+    if (nodes && !mat.cell_control) {
+        PLATO_CUDA(h, launch_pdl(k_cell_nodes, grid_for(h->N, kThreads, 148 * 16), kThreads, h->stream, h->N,
+                                 (const int32_t*)h->n2c_ptr, (const int32_t*)h->n2c, (const double*)h->fans.part, out,
+                                 A.accumulate));
+        PLATO_LAUNCH_CHECK(h);
+    }
+    return fan_end(h);
+}
+
 }  // namespace
 
 // R = K(z) u + scale_F * F: ElastostaticResidual::evaluate (src/elliptic/ElastostaticResidual.hpp:
@@ -508,14 +613,12 @@ int launch_nodal_control_derivative(plato_problem* h, int mode, const double* u,
     A.cell_out = out;
     A.accumulate = accumulate;
     switch (mode) {
-        case 1: PLATO_RC((launch_fans<FAN_QUANT, 1, double>(h, h->material, A, nullptr))); break;
-        case 2: PLATO_RC((launch_fans<FAN_QUANT, 2, double>(h, h->material, A, nullptr))); break;
-        case 3: PLATO_RC((launch_fans<FAN_QUANT, 3, double>(h, h->material, A, nullptr))); break;
-        case 4: PLATO_RC((launch_fans<FAN_QUANT, 4, double>(h, h->material, A, nullptr))); break;
+        case 1: return launch_scalar<FAN_QUANT, 1>(h, h->material, A, out);
+        case 2: return launch_scalar<FAN_QUANT, 2>(h, h->material, A, out);
+        case 3: return launch_scalar<FAN_QUANT, 3>(h, h->material, A, out);
+        case 4: return launch_scalar<FAN_QUANT, 4>(h, h->material, A, out);
         default: return plato_fail(h, PLATO_BAD_INPUT, "unknown control-derivative mode");
     }
-    if (h->material.cell_control) return PLATO_OK;  // the per-cell quantity is the derivative itself
-    return launch_fan_nodes<1, double>(h, out, nullptr, 0.0, accumulate, nullptr, nullptr);
 }
 
 // Internal elastic energy into *result (device scalar).
@@ -525,7 +628,7 @@ int launch_energy(plato_problem* h, const double* u, const double* z, double* re
     A.u = u;
     A.z = z;
     A.result = result;
-    return launch_fans<FAN_QUANT, 0, double>(h, h->material, A, nullptr);
+    return launch_scalar<FAN_QUANT, 0>(h, h->material, A, nullptr);
 }
 
 // Compliance into *result (device scalar) and the self-adjoint dC/dz into dfdz, one pass (what an
@@ -537,9 +640,7 @@ int launch_energy_and_gradient(plato_problem* h, const double* u, const double* 
     A.z = z;
     A.result = result;
     A.cell_out = dfdz;
-    PLATO_RC((launch_fans<FAN_QUANT, 5, double>(h, h->material, A, nullptr)));
-    if (h->material.cell_control) return PLATO_OK;
-    return launch_fan_nodes<1, double>(h, dfdz, nullptr, 0.0, 0, nullptr, nullptr);
+    return launch_scalar<FAN_QUANT, 5>(h, h->material, A, dfdz);
 }
 
 // Geometric "Volume" criterion (src/geometric/Volume.hpp:83-110) with its own penalty, and its derivative.
@@ -548,7 +649,7 @@ int launch_volume(plato_problem* h, const Material& pen, const double* z, double
     A.coords = h->coords_soa;
     A.z = z;
     A.result = result;
-    return launch_fans<FAN_VOLUME, 0, double>(h, pen, A, nullptr);
+    return launch_scalar<FAN_VOLUME, 0>(h, pen, A, nullptr);
 }
 
 int launch_volume_gradient(plato_problem* h, const Material& pen, const double* z, double* dvdz) {
@@ -556,9 +657,7 @@ int launch_volume_gradient(plato_problem* h, const Material& pen, const double* 
     A.coords = h->coords_soa;
     A.z = z;
     A.cell_out = dvdz;
-    PLATO_RC((launch_fans<FAN_VOLUME, 1, double>(h, pen, A, nullptr)));
-    if (pen.cell_control) return PLATO_OK;
-    return launch_fan_nodes<1, double>(h, dvdz, nullptr, 0.0, 0, nullptr, nullptr);
+    return launch_scalar<FAN_VOLUME, 1>(h, pen, A, dvdz);
 }
 
 // ---- matrix-free operator ---------------------------------------------------------------------

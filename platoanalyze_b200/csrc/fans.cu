@@ -186,6 +186,17 @@ __global__ void k_number_axis(int32_t N, const double* __restrict__ x, unsigned 
     }
 }
 
+// *count += the cells whose smallest node number is within 64 of the cell before's
+__global__ void k_cell_steps(int32_t C, const int4* __restrict__ conn, unsigned long long* __restrict__ count) {
+    unsigned int mine = 0;
+    for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c + 1 < C; c += (int64_t)gridDim.x * blockDim.x) {
+        const int4 a = conn[c], b = conn[c + 1];
+        mine += abs(min(min(a.x, a.y), min(a.z, a.w)) - min(min(b.x, b.y), min(b.z, b.w))) <= 64;
+    }
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    if ((threadIdx.x & 31) == 0 && mine) atomicAdd(count, (unsigned long long)mine);
+}
+
 // Sort key of each fan: batch member, then the Morton code of the block its edge midpoint lies in.
 __global__ void k_morton(int32_t nf, const int32_t* __restrict__ nodes, const double* __restrict__ x, double x0,
                          double x1, double x2, double s0, double s1, double s2, const int32_t* __restrict__ member_off,
@@ -360,6 +371,19 @@ int ring_nodes(int64_t cells) {
     return cells < 400 * int64_t(kNumSMs) ? 3 : kRing;
 }
 
+// Whether the scalar quantities (energy, volume, control derivatives) run cell by cell.  On a box cut into Kuhn's six cells,
+// jittered or not, a fan has 5 to 6 cells and shares more than the walk costs; on a general mesh it has about two,
+// and a warp walks as long as its longest fan with a third of the warps.  Jitter of 0.3 of the spacing, 3.6 cells a fan,
+// is about even (120x60x60: dC/dz 86 by fans, 79 us by cells, value and dC/dz 122 and 114, energy 66 and 68, lambda
+// 125 and 96; 5.5 cells: 54 and 78, 85 and 114, 53 and 69, 78 and 96), two cells are not (1.1 M Delaunay cells: dC/dz 56 and 42,
+// lambda 78 and 54, energy 35 and 27, volume gradient 41 and 33).  The cells come in the mesh's order; the
+// fans are sorted by place, so where neighbours in the numbering are far apart the fans win (the same, shuffled: dC/dz 73
+// and 110, lambda 102 and 133).  Below the size at which fans get their full length both take the time of two launches.
+// The residual and the matrix-free product stay with the fans, which win on all of these (1.1 M cells 76 and 94).
+bool cells_win(int64_t cells, int64_t nfans, int64_t close) {
+    return cells >= 400 * int64_t(kNumSMs) && cells < 3 * nfans && 2 * close >= cells;
+}
+
 }  // namespace
 
 void fan_release(plato_problem* h) {
@@ -434,19 +458,21 @@ int fan_plan(plato_problem* h) {
 
     // order by blocks along a Morton curve; within a block the sort keeps the groups' order, by node
     int32_t *order = nullptr, *order_in = nullptr, *members = nullptr;
-    unsigned long long* axis_d = nullptr;
+    unsigned long long* axis_d = nullptr;  // pairs along each axis, and close cells
     const int nmem = h->batch.nseg > 0 ? h->batch.nseg : 1;
     PLATO_CUDA(h, mem.get(&order, nf));
     PLATO_CUDA(h, mem.get(&order_in, nf));
     PLATO_CUDA(h, mem.get(&members, nmem));
-    PLATO_CUDA(h, mem.get(&axis_d, 3));
+    PLATO_CUDA(h, mem.get(&axis_d, 4));
     const int32_t zero = 0;
     PLATO_CUDA(h, cudaMemcpyAsync(members, h->batch.nseg > 0 ? h->batch.node_off.data() : &zero, sizeof(int32_t) * nmem,
                                   cudaMemcpyHostToDevice, s));
-    PLATO_CUDA(h, cudaMemsetAsync(axis_d, 0, 3 * sizeof(unsigned long long), s));
+    PLATO_CUDA(h, cudaMemsetAsync(axis_d, 0, 4 * sizeof(unsigned long long), s));
     k_number_axis<<<grid_for(N, kT, 148 * 8), kT, 0, s>>>(N, h->coords, axis_d);
     PLATO_LAUNCH_CHECK(h);
-    unsigned long long axis[3] = {0, 0, 0};
+    k_cell_steps<<<grid_for(C, kT, 148 * 8), kT, 0, s>>>(C, h->conn, axis_d + 3);
+    PLATO_LAUNCH_CHECK(h);
+    unsigned long long axis[4] = {0, 0, 0, 0};
     PLATO_CUDA(h, cudaMemcpyAsync(axis, axis_d, sizeof(axis), cudaMemcpyDeviceToHost, s));
     PLATO_CUDA(h, cudaStreamSynchronize(s));
     const int along = axis[2] >= axis[1] && axis[2] >= axis[0] ? 2 : (axis[1] >= axis[0] ? 1 : 0);
@@ -501,10 +527,11 @@ int fan_plan(plato_problem* h) {
     PLATO_CUDA(h, cudaStreamSynchronize(s));
     PLATO_CUDA(h, mem.get(&node, ne));
     PLATO_CUDA(h, mem.get(&first, int64_t(ne) + 1));
+    const int by_cell = cells_win(C, nf, int64_t(axis[3]));
     Arena by_entry;
     by_entry.add(&P.place, ne);
     by_entry.add(&P.slot, ne);
-    by_entry.add(&P.part, 3 * int64_t(ne));  // workspace: three values per entry
+    by_entry.add(&P.part, std::max<int64_t>(3 * int64_t(ne), by_cell ? C : 0));  // workspace: three values per entry
     PLATO_CUDA(h, by_entry.allocate(&P.mem[1]));
     k_entries<<<grid_for(int64_t(nv), kT, kGrid), kT, 0, s>>>(int64_t(nv), rkey2, head, entry, nt, P.tile_ptr, node, first,
                                                               count);
@@ -529,6 +556,7 @@ int fan_plan(plato_problem* h) {
 
     PLATO_CUDA(h, cudaStreamSynchronize(s));
     PLATO_CUDA(h, cudaEventCreateWithFlags(&P.end, cudaEventDisableTiming));
+    P.by_cell = by_cell;
     P.nfans = nf;
     P.ntiles = nt;
     P.width = W;

@@ -141,6 +141,7 @@ constexpr int kFanMaxCtas = 148 * 32;  // CTAs of an element kernel
 struct FanPlan {
     int       ready = 0;
     int32_t   nfans = 0, ntiles = 0, width = 0;
+    int       by_cell = 0;  // scalar quantities cell by cell (fans.cu: cells_win)
     void*     mem[2] = {nullptr, nullptr};  // the arrays below, in two allocations (weights apart)
     int32_t*  rec = nullptr;
     int32_t*  cells = nullptr;
@@ -149,7 +150,7 @@ struct FanPlan {
     int32_t*  slot = nullptr;
     uint16_t* inc = nullptr;
     int32_t*  node_ptr = nullptr;
-    double*   part = nullptr;  // [3 * entries] node sums of each tile
+    double*   part = nullptr;  // [3 * entries] node sums of each tile; [cells] quantities of cells (by_cell)
     double*   sums = nullptr;  // [kFanMaxCtas] block sums of the criteria
     double*   w64 = nullptr;   // [6 * nfans] SIMP weight of each cell (matrix-free operator)
     float*    w32 = nullptr;   // the same in FP32

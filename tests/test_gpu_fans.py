@@ -5,6 +5,7 @@ fewer than 100 terms a node and unit-scale data the results agree to 1e-13 relat
 the 1e-11 of the other parity tests."""
 import numpy as np
 import pytest
+from scipy import spatial
 
 from helpers import rel_l2
 from oracle import Oracle
@@ -39,6 +40,24 @@ def shuffled_box(nx, ny, nz, seed):
     return y, np.ascontiguousarray(conn, np.int32)
 
 
+def delaunay(n, shuffle):
+    """About 13 n^3 cells around 2 n^3 jittered lattice points, two to a fan; numbered along the lattice with the
+    cells in the order of their first nodes, or at random.  Cells below 2 % of the lattice's volume are left out:
+    what is left loses two digits at most in its determinants, far inside the bar."""
+    rng = np.random.default_rng(n)
+    g = np.stack(np.meshgrid(np.arange(2 * n), np.arange(n), np.arange(n), indexing="ij"), -1).reshape(-1, 3)
+    x = (g + rng.uniform(-0.3, 0.3, g.shape)) / n
+    conn = spatial.Delaunay(x).simplices
+    v = x[conn]
+    conn = conn[np.abs(np.linalg.det(v[:, :3] - v[:, 3:])) > 0.02 / n ** 3]
+    if not shuffle:
+        return x, np.ascontiguousarray(conn[np.argsort(conn.min(1), kind="stable")], np.int32)
+    perm = rng.permutation(x.shape[0])
+    y = np.empty_like(x)
+    y[perm] = x
+    return y, np.ascontiguousarray(perm[conn][rng.permutation(conn.shape[0])], np.int32)
+
+
 MESHES = {
     "one cell": lambda: (np.array([[0, 0, 0], [1, 0, 0], [0, 1, 0], [0, 0, 1.0]]), np.array([[0, 1, 2, 3]], np.int32)),
     "closed fan of 3": lambda: axis_fan(3, True, 0.2),
@@ -55,6 +74,9 @@ MESHES = {
     "box, tiles of 32 fans": lambda: (lambda m: (m.coords, m.connectivity))(box_mesh(7, 5, 4)),
     "shuffled box, tiles of 32 fans": lambda: shuffled_box(9, 7, 6, 1),
     "shuffled box, tiles of 64 fans": lambda: shuffled_box(40, 33, 30, 2),
+    "Delaunay, scalar quantities by cells": lambda: delaunay(18, False),
+    "Delaunay, shuffled": lambda: delaunay(18, True),
+    "Delaunay, fans of single cells": lambda: delaunay(8, False),
     "box, tiles of 128 fans": lambda: (lambda m: (m.coords, m.connectivity))(box_mesh(51, 39, 39)),
 }
 
@@ -102,6 +124,22 @@ def test_element_kernels(name):
     close(p.vf_value(ud, zed), orc.vf_value(u, ze))
     close(p.sf_gradient_z(ud, zed), orc.sf_gradient_z(u, ze))
     close(np.array([p.sf_value(ud, zed), p.volume_value(zed)]), np.array([orc.sf_value(u, ze), orc.volume_value(ze)]))
+
+
+@pytest.mark.parametrize("name", ["Delaunay, scalar quantities by cells", "box, tiles of 128 fans"])
+def test_element_control_adds(name):
+    """One density per cell: the derivative is added to what is there, by cells and by fans."""
+    x, conn = MESHES[name]()
+    N, C = x.shape[0], conn.shape[0]
+    spec = ProblemSpec(x, conn, 1.7, 0.28, 3.0, 1e-9, [], np.array([0, 1, 5], np.int32), np.zeros(3))
+    p, orc = EllipticProblem(spec), Oracle.from_spec(spec, cell_control=True)
+    p.set_control_layout("element")
+    z = splitmix_uniform(C, 6, 0.3, 1.0)
+    u, start = np.sin(0.3 * np.arange(3 * N) + 0.2), np.cos(0.1 * np.arange(C))
+    # with lambda = u the product is vol eps(u).C.eps(u) s'(rho), twice the energy's derivative
+    want = start + 2.0 * orc.sf_gradient_z(u, z)
+    ud = p.to_dev(u)
+    close(p.vf_gradient_z_apply(ud, p.to_dev(z), ud, p.to_dev(start)), want)
 
 
 @pytest.mark.parametrize("name", MESHES)
