@@ -23,12 +23,15 @@
 // accumulator is [slot][component][lane ^ component]: in the accumulation every lane
 // touches the same component at a time, so the 64-bit accesses of a half warp hit 16
 // distinct bank pairs; in the row-major write-out (CRS) 16 consecutive entries of one row
-// span at most 9 components, two to a bank pair.  The CRS output's transposes and diagonal blocks go out
-// nine lanes to a block as well: a store of one value of 32 blocks touches 32 lines, three whole
-// blocks 3 to 6.  Coordinates are read from planes (a warp's 32 consecutive rows see 2 to 3 lines a load
-// instead of 6).  CRS of 120x60x60: 471 -> 441 us; bound by latency with the 12 warps that the registers
-// allow.  Incidence entries laid out slice-major were slower (491 us): a lane's own entries share
-// a line that stays in L1, a slice's next entries come from L2.
+// span at most 9 components, two to a bank pair.  The CRS output's diagonal blocks, and in a slice whose
+// rows are about as long as one another its transposes, go out nine lanes to a block as well: a store
+// of one value of 32 blocks touches 32 lines, three whole blocks 3 to 6.  CRS of 120x60x60: 467 -> 436 us; bound by
+// latency with the 12 warps that the registers allow.  In a slice of uneven rows, which general meshes have, most
+// of such stores would be empty, and each lane writes its own transposes (1.1 M Delaunay cells: 501 us, 546 with nine lanes;
+// the slices of those fill 0.58 of their longest row, those of a box nearly 1, hence 3/4).  Coordinates read from
+// planes gave nothing on boxes and cost 17 % on a shuffled numbering.  Incidence entries laid out
+// slice-major were slower (491 us): a lane's own entries share a line that stays in L1, a slice's next entries
+// come from L2.
 //
 // Rows with more than kAsmMaxUp upper blocks or more than 255 blocks (high-valence nodes of
 // general meshes) are "wide": skipped here and assembled whole, with the transposes of their
@@ -158,7 +161,7 @@ __device__ __forceinline__ void store_sell(const SellOut& so, int64_t o, double 
 // 9 x 32 x up values and the CTA as many warps as the shared memory takes (at most 14).
 template <bool kSell, typename T>
 __global__ void __launch_bounds__(kAsmMaxWarps * 32, 1)
-k_assemble_rows(MeshView m, const double* __restrict__ px, GraphView g, Material mat, const double* __restrict__ z,
+k_assemble_rows(MeshView m, GraphView g, Material mat, const double* __restrict__ z,
                 const uint16_t* __restrict__ plan, const uint8_t* __restrict__ mirror,
                 const uint8_t* __restrict__ wide, int up, double* __restrict__ crs, SellOut so) {
     const int nwarps = blockDim.x >> 5;
@@ -166,7 +169,6 @@ k_assemble_rows(MeshView m, const double* __restrict__ px, GraphView g, Material
     T* smem = reinterpret_cast<T*>(smem_raw);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     T* acc = smem + warp * (9 * 32 * up);
-    const double *py = px + g.num_nodes, *pz = py + g.num_nodes;  // coordinate planes
     const T lam = T(mat.c01), mu = T(mat.c33);
     const int32_t nslices = (g.num_nodes + 31) >> 5;
     for (int32_t s = blockIdx.x * nwarps + warp; s < nslices; s += gridDim.x * nwarps) {
@@ -181,9 +183,9 @@ k_assemble_rows(MeshView m, const double* __restrict__ px, GraphView g, Material
                 kc = g.n2c_ptr[r + 1] - ks;
                 dslot = g.diag[r] - rs;
                 nup = nb - dslot - 1;
-                xr[0] = T(__ldg(px + r));
-                xr[1] = T(__ldg(py + r));
-                xr[2] = T(__ldg(pz + r));
+                xr[0] = T(__ldg(m.coords + 3 * (int64_t)r));
+                xr[1] = T(__ldg(m.coords + 3 * (int64_t)r + 1));
+                xr[2] = T(__ldg(m.coords + 3 * (int64_t)r + 2));
                 zr = mat.cell_control ? T(0) : T(__ldg(z + r));
             }
         }
@@ -206,9 +208,12 @@ k_assemble_rows(MeshView m, const double* __restrict__ px, GraphView g, Material
             const int32_t i0 = la == 0 ? nk.y : nk.x;
             const int32_t i1 = la <= 1 ? nk.z : nk.y;
             const int32_t i2 = la <= 2 ? nk.w : nk.z;
-            cx[0] = __ldg(px + i0); cx[1] = __ldg(py + i0); cx[2] = __ldg(pz + i0);
-            cx[3] = __ldg(px + i1); cx[4] = __ldg(py + i1); cx[5] = __ldg(pz + i1);
-            cx[6] = __ldg(px + i2); cx[7] = __ldg(py + i2); cx[8] = __ldg(pz + i2);
+            const double* c0 = m.coords + 3 * (int64_t)i0;
+            const double* c1 = m.coords + 3 * (int64_t)i1;
+            const double* c2 = m.coords + 3 * (int64_t)i2;
+            cx[0] = __ldg(c0); cx[1] = __ldg(c0 + 1); cx[2] = __ldg(c0 + 2);
+            cx[3] = __ldg(c1); cx[4] = __ldg(c1 + 1); cx[5] = __ldg(c1 + 2);
+            cx[6] = __ldg(c2); cx[7] = __ldg(c2 + 1); cx[8] = __ldg(c2 + 2);
             if (mat.cell_control) {
                 cz[0] = __ldg(z + (pk >> 2));
                 cz[1] = cz[2] = 0.0;
@@ -365,7 +370,8 @@ k_assemble_rows(MeshView m, const double* __restrict__ px, GraphView g, Material
                 }
             }
         } else {
-            // upper blocks: K back into the accumulator, the transposes straight to row c
+            // upper blocks: K back into the accumulator; in a ragged slice the transposes straight to row c
+            const bool even = 4 * int(__reduce_add_sync(0xffffffffu, unsigned(nup))) >= 3 * 32 * nupw;
             for (int u = 0; u < nup; ++u) {
                 T S[9];
 #pragma unroll
@@ -379,11 +385,21 @@ k_assemble_rows(MeshView m, const double* __restrict__ px, GraphView g, Material
                         K[3 * i + jj] = lam * S[3 * i + jj] + mu * S[3 * jj + i] + (i == jj ? tr : T(0));
 #pragma unroll
                 for (int q = 0; q < 9; ++q) acc[acc_index<kSell>(u, q, lane)] = K[q];
+                if (even) continue;
+                const int k = dslot + 1 + u;
+                const uint8_t ms = __ldg(mirror + rs + k);
+                if (ms != kNoMirror) {
+                    double* dst = crs + 9 * ((int64_t)__ldg(g.row_map + __ldg(g.cols + rs + k)) + ms);
+#pragma unroll
+                    for (int i = 0; i < 3; ++i)
+#pragma unroll
+                        for (int jj = 0; jj < 3; ++jj) dst[3 * i + jj] = double(K[3 * jj + i]);
+                }
             }
             __syncwarp();
-            // the transposes into rows c: nine lanes write a block, three blocks per store
+            // of an even one nine lanes write a block, three blocks per store
             const int wg = lane / 9, wq = lane - 9 * wg, wt = 3 * (wq % 3) + wq / 3;
-            for (int u = 0; u < nupw; ++u) {
+            for (int u = 0; even && u < nupw; ++u) {
                 int32_t blk = -1;  // this row's block in row c
                 if (u < nup) {
                     const int k = dslot + 1 + u;
@@ -476,7 +492,7 @@ int launch_assemble_jacobian(plato_problem* h, const double* z, double* entries)
     int grid = 0, threads = 0, smem = 0;
     PLATO_RC(asm_launch(h, reinterpret_cast<const void*>(k_assemble_rows<false, double>), sizeof(double), &grid,
                         &threads, &smem));
-    k_assemble_rows<false, double><<<grid, threads, smem, h->stream>>>(mesh_view(h), h->coords_soa, graph_view(h), h->material, z,
+    k_assemble_rows<false, double><<<grid, threads, smem, h->stream>>>(mesh_view(h), graph_view(h), h->material, z,
                                                                       h->asm_plan, h->asm_mirror, h->asm_wideflag,
                                                                       h->asm_maxup, entries, SellOut{});
     PLATO_LAUNCH_CHECK(h);
@@ -505,7 +521,7 @@ int launch_assemble_sell(plato_problem* h, const double* z, double* v64, float* 
     SellOut so{h->sell.ptr, h->sell.cols, h->bc_mask, v64, v32, static_cast<__nv_bfloat16*>(v16), dinv, dinv32};
     // the solver's assembly timing (instrumentation) brackets this one kernel
     if (h->timing && h->asm_ev[0]) PLATO_CUDA(h, cudaEventRecord(h->asm_ev[0], h->stream));
-    k_assemble_rows<true, double><<<grid, threads, smem, h->stream>>>(mesh_view(h), h->coords_soa, graph_view(h), h->material, z,
+    k_assemble_rows<true, double><<<grid, threads, smem, h->stream>>>(mesh_view(h), graph_view(h), h->material, z,
                                                                      h->asm_plan, h->asm_mirror, h->asm_wideflag,
                                                                      h->asm_maxup, nullptr, so);
     PLATO_LAUNCH_CHECK(h);
@@ -523,7 +539,7 @@ int launch_assemble_sell32(plato_problem* h, const double* z, float* v32, float*
     PLATO_RC(asm_launch(h, reinterpret_cast<const void*>(k_assemble_rows<true, float>), sizeof(float), &grid,
                         &threads, &smem));
     SellOut so{h->sell.ptr, h->sell.cols, h->bc_mask, nullptr, v32, nullptr, nullptr, dinv32};
-    k_assemble_rows<true, float><<<grid, threads, smem, h->stream>>>(mesh_view(h), h->coords_soa, graph_view(h), h->material, z,
+    k_assemble_rows<true, float><<<grid, threads, smem, h->stream>>>(mesh_view(h), graph_view(h), h->material, z,
                                                                     h->asm_plan, h->asm_mirror, h->asm_wideflag,
                                                                     h->asm_maxup, nullptr, so);
     PLATO_LAUNCH_CHECK(h);
