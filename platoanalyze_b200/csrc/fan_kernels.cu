@@ -307,10 +307,9 @@ k_fans(FanView fv, Material mat, FanArgs<T> A, const PcgScalars* S) {
         double v[1] = {total};
         block_sum_n<1>(v, sh);
         if (publish_partials<1>(v, A.sums, A.ticket, &last)) {
-            double t[1];
-            final_sums<1>(t, A.sums, sh);
+            const double t = final_sum_narrow(A.sums, sh);
             if (tid == 0) {
-                *A.result = t[0];
+                *A.result = t;
                 *A.ticket = 0u;
             }
         }
