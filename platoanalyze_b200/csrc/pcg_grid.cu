@@ -10,11 +10,11 @@
 //   A p with p = z + beta p formed at each gathered column   -> sum p.Ap over the grid -> alpha
 //   x += alpha p, r -= alpha A p, z = Dinv r                 -> sums r.z, r.r          -> beta
 // so two grid-wide sums per iteration, which are also its two barriers.  Only z and p leave the SM.
-// Bound by the two sums (1.5 to 3 us each).  Solve of a cantilever with a random density, launch per stage
-// against this: 20x10x10 15.1 -> 3.2 ms (2.5 as one cluster, see pcg_grid), 30x16x16 24.9 -> 5.2, 40x20x20 30.4 -> 7.5, 60x30x30 54.4 -> 20.6,
-// 64x32x32 84.5 -> 26.4.  Density filter (one unknown per row): 20x10x10 0.66 -> 0.26 ms, 80x40x40
-// 1.92 -> 0.96, 100x50x50 3.30 -> 1.69, 112x53x52 (the largest that qualifies) 4.00 -> 3.81: there the
-// CTAs read the matrix from L2 with two slices per warp, hence the limits in pcg_grid_ok.
+// Bound by the two sums (1.5 to 3 us each).  Solve of a cantilever with a random density to 1e-8, launch per stage
+// against this: 12x6x6 6.9 -> 1.2 ms and 20x10x10 12.7 -> 2.2 (as one cluster, see pcg_split), 30x16x16 19.7 -> 4.6, 40x20x20
+// 24.6 -> 6.3, 60x30x30 42.0 -> 18.1, 64x32x32 70.9 -> 19.6, 72x31x31 (2,336 of the 2,368 slices that qualify) 75.5 ->
+// 28.0.  Density filter (one unknown per row) to 1e-12: 20x10x10 0.74 -> 0.25 ms, 80x40x40 2.77 -> 1.45, 100x50x50 5.34
+// -> 2.57, 106x52x51 (9,217 of 9,472 slices, two to a warp) 5.58 -> 3.17.
 #include <algorithm>
 #include <utility>
 
@@ -272,10 +272,18 @@ int grid_box(plato_problem* h, GridBox* box) {
 // Whether the iterations of this system run in cooperative launches: the device has them, every slice has a
 // group of warps (one slice a group for block systems, at most two for scalar ones), nothing else wants a
 // look between iterations (sampled timings, a deflated direction), and no earlier launch gave up.
+//
+// A scalar system with 17 to 26 slices per SM gives each a warp and leaves the other 6 to 15 of the CTA idle.  With
+// rows as narrow as a box's (15 blocks a slot row) the matrix is in shared memory and that does not matter (72x36x36, 22 slices,
+// shuffled: 28.0 -> 18.6 us an iteration); Delaunay rows (27) are read from L2, and the launch per stage is the steadier
+// one: 17 slices 20.6 us against 23.8, 20 shuffled 30.6 against 36.3, 22 RCM 22.8 against 28.0, shuffled 31.3 against 42, 26 23.8
+// against 25.8 (RCM 26.3 against 23.4).  With 28 and 36 the loop wins again (36.2 -> 31.2, 41.6 -> 35.8 us), as with 16.
 bool pcg_grid_ok(const plato_problem* h, int nb) {
     if (h->grid_off || h->timing || h->ritz_deflating) return false;
-    const int64_t warps = (nb == 3 ? grid_threads<3>() : grid_threads<1>()) / 32;
-    return h->sell.nslices <= int64_t(h->coop_sms) * warps * (nb == 3 ? 1 : 2);
+    const int64_t warps = (nb == 3 ? grid_threads<3>() : grid_threads<1>()) / 32, n = h->sell.nslices;
+    if (n > int64_t(h->coop_sms) * warps * (nb == 3 ? 1 : 2)) return false;
+    const bool wide = h->sell.total_slots > 20 * 32 * n;
+    return !(nb == 1 && wide && n > 16 * int64_t(h->coop_sms) && n <= 26 * int64_t(h->coop_sms));
 }
 
 namespace {

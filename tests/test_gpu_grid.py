@@ -300,3 +300,18 @@ def test_multistep_sweep_on_the_staged_loop(cells):
     for it, u in got[1:]:
         assert it == got[0][0] and rel_l2(u, got[0][1]) <= 1e-14
     assert rel_l2(v.cpu().numpy(), got[0][1]) <= 1e-8
+
+
+@pytest.mark.parametrize("size,mirrored,cooperative", [((72, 36, 35), False, 1), ((72, 36, 35), True, 0), ((90, 40, 38), True, 1)], ids=str)
+def test_filter_of_wide_rows(size, mirrored, cooperative):
+    """21 slices per SM run cooperatively with narrow rows and stay with the launch per stage with wide ones; 31 slices
+    of wide rows per SM, two to a warp and read from L2, run cooperatively.  The bars of the other comparisons."""
+    m, conn = mirrored_box(*size)
+    f = HelmholtzFilter(m.coords, conn if mirrored else m.connectivity, 0.08)
+    c = f.to_dev(splitmix_uniform(m.num_nodes, 4))
+    a, sa = f.solution(c)
+    used = np.zeros(1, np.int32)
+    assert capi.lib.plato_get_loop_info(f.h, used.ctypes.data_as(capi.i32p)) == capi.OK and used[0] == cooperative
+    f.set_timing(True)
+    b, sb = f.solution(c)
+    assert abs(sa["iterations"] - sb["iterations"]) <= 2 and rel_l2(a.cpu().numpy(), b.cpu().numpy()) <= 1e-10
