@@ -16,8 +16,8 @@
 // lambda_max comes from a few Lanczos steps with a safety factor.
 //
 // Each Chebyshev step on the SELL copy is one fused kernel (gather SpMV, residual update,
-// direction and iterate update; no reductions).  The matrix-free variant scatters with
-// FP32 atomics and finishes the step in a vector kernel.
+// direction and iterate update; no reductions).  The matrix-free variant applies the FP32 operator
+// with the fan kernels (fan_kernels.cu: fixed-order sums, no atomics) and finishes the step in a vector kernel.
 #include <algorithm>
 #include <cmath>
 #include <cuda_bf16.h>

@@ -11,7 +11,7 @@
 //    channels, K = taps x input channels, on tcgen05 with FP32 accumulators in tensor memory:
 //    k_conv_tz marches along z and uses each input plane for three output planes, k_conv_tc
 //    takes the layers whose weights it cannot keep beside its slabs (96 -> 32, 64 -> 64), those of
-//    more than 80 output channels and the 1x1x1 head.  k_conv (mma.sync, A fragments gathered from the haloed
+//    more than 64 output channels and the 1x1x1 head.  k_conv (mma.sync, A fragments gathered from the haloed
 //    tensor) is the second family of the API.  Bias, ReLU and FP32 accumulation are fused in
 //    the epilogue.  The data gradient is the same convolution with flipped, transposed weights.
 //  * Weight gradient: GEMM over voxels, M = output channels, N = input channels, K =
@@ -581,6 +581,12 @@ template <int COUTP>
 constexpr int tz_tmem_cols() {
     return tz_ring<COUTP>() * COUTP <= 128 ? 128 : 256;
 }
+// the widths whose ring fits in those columns (and whose three weight blocks in one MMA): up to 64 channels
+template <int COUTP>
+constexpr bool tz_width() {
+    return 3 * COUTP <= 256 && tz_ring<COUTP>() * COUTP <= tz_tmem_cols<COUTP>();
+}
+static_assert(tz_width<16>() && tz_width<32>() && tz_width<48>() && tz_width<64>() && !tz_width<80>(), "ring widths");
 
 struct TzGeom {
     int32_t  ncol;    // columns of 128 positions per plane
@@ -605,7 +611,7 @@ __global__ void __launch_bounds__(128)
 k_conv_tz(TView in, const bf16* __restrict__ Wt, const float* __restrict__ bias, TView out, TzGeom g,
           int* __restrict__ err) {
     constexpr int COUTP = (COUT + 15) / 16 * 16;
-    static_assert(CIN % 16 == 0 && COUT % 16 == 0 && 3 * COUTP <= 256, "UMMA shape");
+    static_assert(CIN % 16 == 0 && COUT % 16 == 0 && tz_width<COUTP>(), "UMMA shape, columns of the ring");
     constexpr bool SW = CIN == 16;  // 16-channel slabs: rows of 32 B in the 32-byte swizzle
     constexpr int R = tz_ring<COUTP>();
     constexpr uint32_t BTAP = 3u * COUTP * CIN * 2;           // one (dy, dx) tap: the weights of three dz
@@ -1618,7 +1624,7 @@ int conv_launch(cudaStream_t s, const ConvPath& P, TView in, const bf16* w, cons
         constexpr int COUTP = (COUT + 15) / 16 * 16;
         const int64_t sy = in.W + 2, sz = int64_t(in.H + 2) * sy;
         const int64_t ptotal = int64_t(in.B) * (in.D + 2) * sz;
-        if constexpr (TAPS == 27 && COUT % 16 == 0 && 3 * COUT <= 256) {
+        if constexpr (TAPS == 27 && COUT % 16 == 0 && tz_width<COUT>()) {
             TzGeom tz{};
             uint32_t tz_smem = 0;
             int tz_grid = 0;
