@@ -318,19 +318,21 @@ k_fans(FanView fv, Material mat, FanArgs<T> A, const PcgScalars* S) {
 
 // A scalar quantity cell by cell, a thread each, where the fans are short (cells_win in fans.cu): the derivative per
 // cell goes to cell_out (one density per cell) or to part, from where k_cell_nodes sums it per node.  Four CTAs an SM at 64
-// registers hide the 14 to 40 gathers of a cell, which bound it: kernels of 1.1 M Delaunay cells, dC/dz 24.7 + 17.0
-// us, (dR/dz)^T lambda 36.1 + 17.3 us (a fan with its 168 registers: 55 and 77 us together).
+// registers (three with lambda, where four spill: 35.5 -> 33.8 us) hide the 14 to 40 gathers of a cell, which bound it.  Its edges start from the corner that a fan's do, the
+// end of its longest edge: a sliver's determinant depends on that (error of a lambda product on 77,101 Delaunay cells against
+// extended precision 8e-16, from the first corner 6.6e-15).  Measured: kernels of 1.1 M Delaunay cells, dC/dz 24.0 + 17.0
+// us, (dR/dz)^T lambda 33.8 + 17.3 us (a fan with its 168 registers: 55 and 77 us together), energy 25.6 us (36).
 constexpr int kCellThreads = 256;
 template <int OP, int MODE>
-__global__ void __launch_bounds__(kCellThreads, 4)
-k_cells(int32_t C, const int4* __restrict__ conn, const double* __restrict__ coords, Material mat, FanArgs<double> A) {
+__global__ void __launch_bounds__(kCellThreads, fan_has_lam<OP, MODE>() ? 3 : 4)
+k_cells(int32_t C, const int4* __restrict__ corners, const double* __restrict__ coords, Material mat, FanArgs<double> A) {
     constexpr bool U = fan_has_u<OP>(), L = fan_has_lam<OP, MODE>();
     constexpr bool NODES = fan_nodes<OP, MODE>(), SUMS = fan_sums<OP, MODE>();
     double total = 0.0;
     double* out = mat.cell_control ? A.cell_out : A.part;
     const bool add = mat.cell_control && A.accumulate;
     for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < C; c += (int64_t)gridDim.x * blockDim.x) {
-        const int4 n = __ldg(conn + c);
+        const int4 n = __ldg(corners + c);
         auto at = [](const double* v, int64_t a) { return Vec3<double>{__ldg(v + 3 * a), __ldg(v + 3 * a + 1), __ldg(v + 3 * a + 2)}; };
         const Vec3<double> xa = at(coords, n.x);
         const Vec3<double> eb = at(coords, n.y) - xa, ep = at(coords, n.z) - xa, en = at(coords, n.w) - xa;
@@ -568,12 +570,12 @@ int launch_scalar(plato_problem* h, const Material& mat, FanArgs<double> A, doub
     A.part = h->fans.part;
     A.sums = h->fans.sums;
     A.ticket = h->red_ticket;
-    // a sum takes one resident wave, whose last CTA then has few block sums to add (energy of 1.1 M cells 26.7 us, 36 with
+    // a sum takes one resident wave, whose last CTA then has few block sums to add (energy of 1.1 M cells 27 us, 36 with
     // a CTA for every 256 cells)
     int wave = kFanMaxCtas;
     if (fan_sums<OP, MODE>())
         PLATO_RC(resident_ctas(h, reinterpret_cast<const void*>(k_cells<OP, MODE>), kCellThreads, 0, &wave));
-    k_cells<OP, MODE><<<grid_for(h->C, kCellThreads, wave), kCellThreads, 0, h->stream>>>(h->C, h->conn, h->coords, mat, A);
+    k_cells<OP, MODE><<<grid_for(h->C, kCellThreads, wave), kCellThreads, 0, h->stream>>>(h->C, reinterpret_cast<const int4*>(h->fans.corners), h->coords, mat, A);
     PLATO_LAUNCH_CHECK(h);
     if (nodes && !mat.cell_control) {
         PLATO_CUDA(h, launch_pdl(k_cell_nodes, grid_for(h->N, kThreads, 148 * 16), kThreads, h->stream, h->N,

@@ -240,6 +240,18 @@ __global__ void k_place(int32_t nf, int32_t width, int32_t ntiles, const int32_t
     }
 }
 
+// The cells' nodes in the order in which the fans take them: the ends of the longest edge, then the two ring nodes, the
+// smaller first (neighbouring cells' nodes then lie side by side more often: energy of 1.1 M cells 28.3 -> 25.6 us).
+__global__ void k_corners(int32_t nf, const int32_t* __restrict__ rec, const int32_t* __restrict__ cells, int4* __restrict__ corners) {
+    for (int64_t f = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; f < nf; f += (int64_t)gridDim.x * blockDim.x) {
+        const int32_t* r = rec + 8 * f;
+        for (int i = 0; i < 6 && cells[6 * f + i] >= 0; ++i) {
+            const int32_t next = i < 5 && r[3 + i] >= 0 ? r[3 + i] : r[2];  // a closed fan's last cell ends at the first ring node
+            corners[cells[6 * f + i]] = make_int4(r[0] & ~kFanClosed, r[1], min(r[2 + i], next), max(r[2 + i], next));
+        }
+    }
+}
+
 __global__ void k_heads(int64_t nref, const uint64_t* __restrict__ key, int32_t ntiles, int32_t* __restrict__ head,
                         unsigned long long* __restrict__ nvalid) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nref; i += (int64_t)gridDim.x * blockDim.x) {
@@ -531,6 +543,7 @@ int fan_plan(plato_problem* h) {
     Arena by_entry;
     by_entry.add(&P.place, ne);
     by_entry.add(&P.slot, ne);
+    by_entry.add(&P.corners, by_cell ? 4 * int64_t(C) : 0);
     by_entry.add(&P.part, std::max<int64_t>(3 * int64_t(ne), by_cell ? C : 0));  // workspace: three values per entry
     PLATO_CUDA(h, by_entry.allocate(&P.mem[1]));
     k_entries<<<grid_for(int64_t(nv), kT, kGrid), kT, 0, s>>>(int64_t(nv), rkey2, head, entry, nt, P.tile_ptr, node, first,
@@ -539,6 +552,11 @@ int fan_plan(plato_problem* h) {
     k_uses<<<grid_for(int64_t(nv), kT, kGrid), kT, 0, s>>>(int64_t(nv), W, rkey2, ref2, head, entry, P.tile_ptr, first,
                                                            P.place, P.inc);
     PLATO_LAUNCH_CHECK(h);
+
+    if (by_cell) {
+        k_corners<<<grid_for(nf, kT, kGrid), kT, 0, s>>>(nf, P.rec, P.cells, reinterpret_cast<int4*>(P.corners));
+        PLATO_LAUNCH_CHECK(h);
+    }
 
     // places of the entries in node order
     uint32_t *ekey = nullptr, *ekey2 = nullptr;
