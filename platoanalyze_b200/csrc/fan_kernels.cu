@@ -318,10 +318,9 @@ k_fans(FanView fv, Material mat, FanArgs<T> A, const PcgScalars* S) {
 
 // A scalar quantity cell by cell, a thread each, where the fans are short (cells_win in fans.cu): the derivative per
 // cell goes to cell_out (one density per cell) or to part, from where k_cell_nodes sums it per node.  Four CTAs an SM at 64
-// registers (three with lambda, where four spill: 35.5 -> 33.8 us) hide the 14 to 40 gathers of a cell, which bound it.  Its edges start from the corner that a fan's do, the
-// end of its longest edge: a sliver's determinant depends on that (error of a lambda product on 77,101 Delaunay cells against
-// extended precision 8e-16, from the first corner 6.6e-15).  Measured: kernels of 1.1 M Delaunay cells, dC/dz 24.0 + 17.0
-// us, (dR/dz)^T lambda 33.8 + 17.3 us (a fan with its 168 registers: 55 and 77 us together), energy 25.6 us (36).
+// registers (three with lambda, where four spill: 35.5 -> 33.8 us) hide the 14 to 40 gathers of a cell, which bound it.  `corners` has each cell's nodes in an order that suits the
+// rounding and the gathers (fans.cu).  Kernels of 1.1 M Delaunay cells: dC/dz 23.2 + 17.0 us, (dR/dz)^T lambda 33.5 + 17.3 us (a
+// fan with its 168 registers: 55 and 77 us together), energy 24.6 us (36).
 constexpr int kCellThreads = 256;
 template <int OP, int MODE>
 __global__ void __launch_bounds__(kCellThreads, fan_has_lam<OP, MODE>() ? 3 : 4)
@@ -570,7 +569,7 @@ int launch_scalar(plato_problem* h, const Material& mat, FanArgs<double> A, doub
     A.part = h->fans.part;
     A.sums = h->fans.sums;
     A.ticket = h->red_ticket;
-    // a sum takes one resident wave, whose last CTA then has few block sums to add (energy of 1.1 M cells 27 us, 36 with
+    // a sum takes one resident wave, whose last CTA then has few block sums to add (energy of 1.1 M cells 25 us, 36 with
     // a CTA for every 256 cells)
     int wave = kFanMaxCtas;
     if (fan_sums<OP, MODE>())

@@ -150,7 +150,7 @@ struct FanPlan {
     int32_t*  slot = nullptr;
     uint16_t* inc = nullptr;
     int32_t*  node_ptr = nullptr;
-    int32_t*  corners = nullptr;  // [4 * cells] each cell's nodes in its fan's order (by_cell)
+    int32_t*  corners = nullptr;  // [4 * cells] each cell's nodes, its corner with the shortest edges first (by_cell)
     double*   part = nullptr;  // [3 * entries] node sums of each tile; [cells] quantities of cells (by_cell)
     double*   sums = nullptr;  // [kFanMaxCtas] block sums of the criteria
     double*   w64 = nullptr;   // [6 * nfans] SIMP weight of each cell (matrix-free operator)
