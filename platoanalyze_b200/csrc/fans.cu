@@ -336,8 +336,10 @@ struct Scratch {
     cudaStream_t s;
     std::vector<void*> held;
     explicit Scratch(plato_problem* handle) : h(handle), s(handle->stream) {}
-    ~Scratch() {
+    ~Scratch() { release(); }
+    void release() {
         for (void* p : held) cudaFreeAsync(p, s);
+        held.clear();
     }
     template <typename T>
     cudaError_t get(T** p, int64_t count) {
@@ -439,47 +441,47 @@ int fan_plan(plato_problem* h) {
     if (P.ready) return PLATO_OK;
     fan_release(h);  // what an earlier attempt that failed has left
     cudaStream_t s = h->stream;
-    Scratch mem(h);
+    Scratch mem(h), early(h);
     const int32_t C = h->C, N = h->N;
     constexpr int kGrid = 148 * 64;
 
     // groups of cells with the same longest edge
     uint64_t *key = nullptr, *key2 = nullptr, *gkey = nullptr;
     int32_t *cell = nullptr, *cell2 = nullptr, *gcount = nullptr, *gstart = nullptr, *ngroups_d = nullptr;
-    PLATO_CUDA(h, mem.get(&key, C));
-    PLATO_CUDA(h, mem.get(&key2, C));
-    PLATO_CUDA(h, mem.get(&gkey, C));
-    PLATO_CUDA(h, mem.get(&cell, C));
-    PLATO_CUDA(h, mem.get(&cell2, C));
-    PLATO_CUDA(h, mem.get(&gcount, C));
-    PLATO_CUDA(h, mem.get(&gstart, C));
-    PLATO_CUDA(h, mem.get(&ngroups_d, 1));
+    PLATO_CUDA(h, early.get(&key, C));
+    PLATO_CUDA(h, early.get(&key2, C));
+    PLATO_CUDA(h, early.get(&gkey, C));
+    PLATO_CUDA(h, early.get(&cell, C));
+    PLATO_CUDA(h, early.get(&cell2, C));
+    PLATO_CUDA(h, early.get(&gcount, C));
+    PLATO_CUDA(h, early.get(&gstart, C));
+    PLATO_CUDA(h, early.get(&ngroups_d, 1));
     k_longest_edge<<<grid_for(C, kT, kGrid), kT, 0, s>>>(C, h->conn, h->coords, key, cell);
     PLATO_LAUNCH_CHECK(h);
-    PLATO_CUDA(h, sort_pairs(mem, key, key2, cell, cell2, C, 32 + bits_for(N)));
+    PLATO_CUDA(h, sort_pairs(early, key, key2, cell, cell2, C, 32 + bits_for(N)));
     {
         size_t bytes = 0;
         char* tmp = nullptr;
         PLATO_CUDA(h, cub::DeviceRunLengthEncode::Encode(nullptr, bytes, key2, gkey, gcount, ngroups_d, C, s));
-        PLATO_CUDA(h, mem.get(&tmp, int64_t(bytes)));
+        PLATO_CUDA(h, early.get(&tmp, int64_t(bytes)));
         PLATO_CUDA(h, cub::DeviceRunLengthEncode::Encode(tmp, bytes, key2, gkey, gcount, ngroups_d, C, s));
     }
     int32_t ng = 0;
     PLATO_CUDA(h, cudaMemcpyAsync(&ng, ngroups_d, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
     PLATO_CUDA(h, cudaStreamSynchronize(s));
-    PLATO_CUDA(h, scan<false>(mem, gcount, gstart, ng));
+    PLATO_CUDA(h, scan<false>(early, gcount, gstart, ng));
 
     // fans of each group: count, place, write
     const int ring_max = ring_nodes(C);
     int32_t *gfans = nullptr, *gfirst = nullptr, *fnodes = nullptr, *fcells = nullptr;
     uint8_t* closed = nullptr;
-    PLATO_CUDA(h, mem.get(&gfans, int64_t(ng) + 1));
-    PLATO_CUDA(h, mem.get(&gfirst, int64_t(ng) + 1));
+    PLATO_CUDA(h, early.get(&gfans, int64_t(ng) + 1));
+    PLATO_CUDA(h, early.get(&gfirst, int64_t(ng) + 1));
     PLATO_CUDA(h, cudaMemsetAsync(gfans + ng, 0, sizeof(int32_t), s));
     k_chain<0><<<grid_for(ng, 128, kGrid), 128, 0, s>>>(ng, ring_max, gkey, gstart, gcount, cell2, h->conn, nullptr, gfans, nullptr,
                                                         nullptr, nullptr);
     PLATO_LAUNCH_CHECK(h);
-    PLATO_CUDA(h, scan<false>(mem, gfans, gfirst, int64_t(ng) + 1));
+    PLATO_CUDA(h, scan<false>(early, gfans, gfirst, int64_t(ng) + 1));
     int32_t nf = 0;
     PLATO_CUDA(h, cudaMemcpyAsync(&nf, gfirst + ng, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
     PLATO_CUDA(h, cudaStreamSynchronize(s));
@@ -495,9 +497,9 @@ int fan_plan(plato_problem* h) {
     unsigned long long* axis_d = nullptr;  // pairs along each axis, and close cells
     const int nmem = h->batch.nseg > 0 ? h->batch.nseg : 1;
     PLATO_CUDA(h, mem.get(&order, nf));
-    PLATO_CUDA(h, mem.get(&order_in, nf));
-    PLATO_CUDA(h, mem.get(&members, nmem));
-    PLATO_CUDA(h, mem.get(&axis_d, 4));
+    PLATO_CUDA(h, early.get(&order_in, nf));
+    PLATO_CUDA(h, early.get(&members, nmem));
+    PLATO_CUDA(h, early.get(&axis_d, 4));
     const int32_t zero = 0;
     PLATO_CUDA(h, cudaMemcpyAsync(members, h->batch.nseg > 0 ? h->batch.node_off.data() : &zero, sizeof(int32_t) * nmem,
                                   cudaMemcpyHostToDevice, s));
@@ -522,7 +524,8 @@ int fan_plan(plato_problem* h) {
     k_morton<<<grid_for(nf, kT, kGrid), kT, 0, s>>>(nf, fnodes, h->coords, h->bbox_min[0], h->bbox_min[1], h->bbox_min[2],
                                                     scale[0], scale[1], scale[2], members, nmem, key, order_in);
     PLATO_LAUNCH_CHECK(h);
-    PLATO_CUDA(h, sort_pairs(mem, key, key2, order_in, order, nf, 30 + bits_for(nmem)));
+    PLATO_CUDA(h, sort_pairs(early, key, key2, order_in, order, nf, 30 + bits_for(nmem)));
+    early.release();  // a general mesh would need 60 bytes a cell more at the references' sort
 
     // tiles: references sorted by (tile, node), and their distinct nodes
     const int32_t W = tile_width(nf), nt = (nf + W - 1) / W;
