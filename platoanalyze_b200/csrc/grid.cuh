@@ -31,14 +31,14 @@ __device__ __forceinline__ void grid_fence() { asm volatile("fence.acq_rel.gpu;"
 
 // Thread 0 of a CTA whose other threads' writes a __syncthreads() has put before this.
 __device__ __forceinline__ bool grid_arrive_and_wait(const GridBox& a, uint32_t barrier) {
-    const bool stalled = barrier == a.stall_barrier && int(blockIdx.x) == a.stall_cta;
-    const uint32_t target = barrier * gridDim.x + (stalled ? 1u << 30 : 0u);
+    uint32_t target = barrier * gridDim.x;
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.count) : "memory");
+    if (barrier == a.stall_barrier && int(blockIdx.x) == a.stall_cta) target += 1u << 30;
     for (uint32_t polls = 1;; ++polls) {
         uint32_t v;
         asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.count) : "memory");
         if (int32_t(v - target) >= 0) break;
-        if (polls > a.polls || ((polls & 1023u) == 0 && *reinterpret_cast<volatile int32_t*>(a.abort))) {
+        if ((polls & 1023u) == 0 && (polls >= a.polls || *reinterpret_cast<volatile int32_t*>(a.abort))) {
             *reinterpret_cast<volatile int32_t*>(a.abort) = 1;
             return false;
         }
