@@ -1566,6 +1566,18 @@ bool tc_plan(int rows, TcGeom& g, uint32_t& smem, int& ctas_per_sm) {
     return true;
 }
 
+// Tiles of 128 positions per SM from which marching along z wins, in hundredths.  Below, k_conv_tc has each tile's 27 taps done
+// by a CTA of its own while a marching CTA walks three planes for one, after clearing its accumulators; the fewer
+// MMAs a tile has (input channels) the later that turns.  us of k_conv_tc and k_conv_tz on both sides (tiles per SM):
+// 16 -> 16 (3.7) 13.5 14.6, (4.6) 21.5 17.9; 32 -> 16 (2.9) 19.9 21.7, (4.3) 26.8 23.7; 48 -> 16 (1.8) 22.0 23.3, (2.2) 27.7 23.1;
+// 16 -> 48 (1.8) 17.0 17.4, (2.2) 18.4 17.7; 32 -> 32 (1.05) 16.6 18.0, (1.09) 17.4 15.2, (1.4) 17.7 19.3, (2.2) 27.5 21.3;
+// 16 -> 32 (1.05) 11.4 11.6, (1.09) 11.9 11.1; 96 -> 32 (0.8) 26.3 27.5, (1.05) 39.1 30.3; 32 -> 64 (0.9) 17.1 19.2,
+// (1.3) 23.7 21.3; 64 -> 32 (0.9) 20.6 22.6, (1.3) 30.1 25.4.  Forward pass at 17x9x9: 176 -> 165 us.
+template <int CIN, int COUT>
+constexpr int tz_from() {
+    return COUT == 16 && CIN <= 32 ? 420 : CIN == 48 || COUT == 48 ? 200 : CIN + COUT <= 64 ? 106 : 100;
+}
+
 // Shared memory, pipeline and runs of a k_conv_tz launch: all weights resident beside 2 to 4 slab
 // buffers, and the number of runs per column that lets the most loaded CTA walk the fewest planes (a
 // run reads two planes more than it writes).  False when the weights do not fit.
@@ -1628,7 +1640,9 @@ int conv_launch(cudaStream_t s, const ConvPath& P, TView in, const bf16* w, cons
             TzGeom tz{};
             uint32_t tz_smem = 0;
             int tz_grid = 0;
-            if (ptotal < (int64_t(1) << 31) && tz_plan<CIN, COUTP>(in, ptotal, tz, tz_smem, tz_grid)) {
+            const int64_t tiles = int64_t(in.B) * in.D * sz / kTcRows;
+            if (ptotal < (int64_t(1) << 31) && 100 * tiles >= int64_t(tz_from<CIN, COUT>()) * sm_count() &&
+                tz_plan<CIN, COUTP>(in, ptotal, tz, tz_smem, tz_grid)) {
                 auto kernel = k_conv_tz<CIN, COUT, RELU, F32, ACC>;
                 UCUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(tz_smem)));
                 kernel<<<tz_grid, 128, tz_smem, s>>>(in, w, b, out, tz, P.err);

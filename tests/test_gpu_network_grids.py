@@ -33,3 +33,18 @@ def test_families_agree(nodes, batch):
         assert abs(again - loss) <= 1e-6 * loss and np.array_equal(net.forward(inp).cpu().numpy(), out)
     (a, la, ga), (b, lb, gb) = got
     assert rel_l2(a, b) <= 5e-3 and rel_l2(ga, gb) <= 1e-2 and abs(la - lb) <= 5e-3 * lb
+
+
+@pytest.mark.parametrize("nodes,batch", [((33, 17, 17), 8), ((20, 33, 33), 3), ((65, 33, 33), 2)])
+def test_a_member_does_not_depend_on_its_batch(nodes, batch):
+    """A batch large enough for the convolutions that march along z against its members one by one, which are
+    not (or, on the largest grid, are in the first layers only): the bar of the families above."""
+    rng = np.random.default_rng(9)
+    nn = int(np.prod(nodes))
+    inp = torch.tensor(rng.uniform(-1, 1, (batch, nn, 8)), dtype=torch.float32).cuda()
+    net = UNet(nodes, batch)
+    net.set_params(init_params(net.num_params, 5))
+    whole = net.forward(inp).cpu().numpy()
+    for k in range(batch):
+        assert rel_l2(net.forward(inp[k:k + 1].contiguous()).cpu().numpy()[0], whole[k]) <= 5e-3
+    net.check()
