@@ -12,9 +12,9 @@
 // form, and the correction Z E^-1 Z^T of it takes five more barriers: restriction per coarse cell (a
 // warp each), its sums, the two triangular products (a warp per row), and the prolongation onto the
 // CTA's own rows.  Bound by these barriers (1.5 to 3 us each) and, beyond what shared memory holds, by L2.
-// Solve, launch per stage against this: FP32 Chebyshev 20x10x10 9.5 -> 3.3 ms, 64x32x32 36.9 -> 19.8;
-// two-level FP32 5.0 -> 2.2 and 10.6 -> 6.0 ms; two-level FP16 5.1 -> 2.2 and 9.2 -> 4.7 ms.  Larger systems
-// have more slices than warps (64x32x32 has 2,244 slices for 2,368 warps) and keep the launch per stage,
+// Solve to 1e-8, launch per stage against this: FP32 Chebyshev 20x10x10 6.9 -> 2.5 ms, 64x32x32 30.1 -> 17.3;
+// two-level FP32 4.0 -> 1.7 and 8.3 -> 4.9 ms; two-level FP16 3.9 -> 1.7 and 7.6 -> 4.0 ms.  64x32x32 has 2,213 slices and
+// 72x31x31 2,336; larger systems have more slices than the 2,368 warps and keep the launch per stage,
 // whose streams from HBM hide its gaps.
 #include <algorithm>
 #include <cuda_bf16.h>

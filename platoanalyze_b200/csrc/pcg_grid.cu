@@ -303,7 +303,7 @@ PcgSplit pcg_split(int nslices, int64_t total_slots, int nb, int sms, bool may_c
     // shared memory for the average CTA's slots and a tenth more; a CTA with more reads L2
     const auto smem_for = [&](int ctas) { return (total_slots / ctas + 32) * (8 * nb * nb + 4) * 11 / 10; };
     // A system that gives each of 16 SMs its part in shared memory and each slice 3 warps (scalar: one) runs
-    // as one cluster, whose barrier is a hardware one.  One grid-wide counter against this: 12x6x6 2.0 -> 1.4 ms,
+    // as one cluster, whose barrier is a hardware one.  One grid-wide counter against this (densities of 0.01 to 1, to 1e-10): 12x6x6 2.0 -> 1.4 ms,
     // 18x9x9 3.0 -> 2.3, 20x10x10 (80 slices, 3 warps each) 3.2 -> 2.5; with 2 warps a slice 21x10x10 3.38 -> 3.41,
     // so the line lies there.  Filter: 16x8x8 0.49 -> 0.38 ms, 37x20x18 (474 slices, a warp each) 0.97 -> 0.86.
     int cluster = 1;
