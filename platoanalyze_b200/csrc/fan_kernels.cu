@@ -552,7 +552,7 @@ int launch_fan_nodes(plato_problem* h, T* out, const T* F, T scale, int accumula
                              (const int32_t*)h->fans.node_ptr, reinterpret_cast<const T*>(h->fans.part), out, F, scale,
                              accumulate, (const uint8_t*)h->bc_mask, copy, S));
     PLATO_LAUNCH_CHECK(h);
-    return fan_end(h);
+    return S ? PLATO_OK : fan_end(h);  // a solver's products: the solve ends with the stream waited for
 }
 
 // A scalar quantity, by fans or by cells; with one density per node its nodal sums go to `out`, or are added to it.
