@@ -253,6 +253,7 @@ struct plato_problem {
     double* K = nullptr;           // 9*nblocks
     double* KT = nullptr;          // scratch for transposed / gradient_z matrices
     // PCG work vectors (3N each) and scalars
+    double* v_mem = nullptr;       // the allocation of F and the vectors below
     double* v_r = nullptr;
     double* v_z = nullptr;
     double* v_p = nullptr;
